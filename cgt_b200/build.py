@@ -9,12 +9,15 @@ import os
 import os.path as osp
 import subprocess
 import sys
+import sysconfig
 
 HERE = osp.dirname(osp.abspath(__file__))
 CSRC = osp.join(HERE, "csrc")
 INCLUDE = osp.join(HERE, "..", "include")
 OBJDIR = osp.join(HERE, "csrc", "build")
 LIB = osp.join(HERE, "libcgt_b200.so")
+BRIDGE_SRC = osp.join(CSRC, "pybridge.cpp")
+BRIDGE = osp.join(HERE, "_pybridge.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -73,6 +76,13 @@ def build(force=False, verbose=False):
         if p.returncode != 0:
             sys.stderr.write(p.stdout + p.stderr)
             raise RuntimeError("link failed")
+    if force or _stale(BRIDGE, [BRIDGE_SRC, osp.join(INCLUDE, "cgt_b200.h")]):
+        cmd = ["c++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-I" + sysconfig.get_paths()["include"], BRIDGE_SRC,
+               "-o", BRIDGE, "-L" + HERE, "-l:libcgt_b200.so", "-Wl,-rpath,$ORIGIN"]
+        p = subprocess.run(cmd, capture_output=True, text=True)
+        if p.returncode != 0:
+            sys.stderr.write(p.stdout + p.stderr)
+            raise RuntimeError("building _pybridge.so failed")
     return LIB
 
 

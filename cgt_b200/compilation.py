@@ -2231,7 +2231,7 @@ def create_interpreter(inputs, outputs, eg, node2memloc):
         flags |= runtime.INTERP_CUDA_GRAPHS
     if config["profile"] or profiler.on:
         flags |= runtime.INTERP_PROFILE
-    interp = runtime.InterpreterWrapper(eg, input_types, output_locs, flags)
+    interp = runtime.InterpreterWrapper(eg, input_types, output_locs, flags, tuple_outputs=any(is_tuple(o) for o in outputs))
     interp.eg = eg
     if flags & runtime.INTERP_PROFILE:
         profiler.register(interp)

@@ -6,8 +6,11 @@
 //
 //   * every device instruction enqueues kernels on the runtime's CUDA stream and returns at once;
 //   * cross-device copies (Transport) are asynchronous; a host instruction that reads array data
-//     waits for the stream only when a device->host copy is outstanding;
-//   * the instruction list is cut into spans at every Transport / non-capturable instruction. Once a
+//     waits for the stream only when a device->host copy is outstanding. The small arrays that a span takes from
+//     the host, the call's arguments that already are on the device among them, are brought to their buffers by ONE
+//     kernel at the span's start, what it hands to the host (the function's results at the end) leaves by one kernel
+//     at its end; both are nodes of the span's graph (host_copy.cu);
+//   * the instruction list is cut into spans after device->host copies and at every non-capturable instruction. Once a
 //     span has run twice with identical buffer addresses (steady state: no allocation happens any
 //     more), its device instructions are captured into a CUDA graph and later runs replay the graph
 //     with one launch. The replay is used only while a key over all buffer addresses and small host
@@ -21,7 +24,9 @@
 //     before, the rest of the run takes the full path again. Without this the host walks the whole instruction
 //     list before each launch: thousands of instructions for an unrolled recurrent network, more time than
 //     the device needs for them.
+#include "host_copy.h"
 #include "runtime.h"
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cstdlib>
@@ -34,7 +39,7 @@ using namespace cgtb;
 namespace {
 
 enum Kind { kLoadArgument, kAlloc, kBuildTup, kReturnByRef, kReturnByVal };
-enum Klass { kMeta, kHostData, kDevice, kBarrier };
+enum Klass { kMeta, kHostData, kDevice, kBarrier, kUpload, kDownload };
 
 struct Loc {
   long idx;
@@ -55,6 +60,8 @@ struct Instr {
   bool fired = false;
   bool arg_view = false;  // host bookkeeping on (a view of) an argument: fired in steady runs too
   ScratchOwner scratch;
+  void* stage = nullptr;  // kUpload: pinned copy of the host operand, read by the span's copy kernel
+  long stage_cap = 0;
   double prof_ms = 0;
   long prof_count = 0;
 };
@@ -62,8 +69,15 @@ struct Instr {
 struct Span {
   int begin = 0, end = 0;  // [begin, end)
   bool barrier = false;    // single Transport / non-capturable instruction
-  int n_device = 0;
+  int n_device = 0;        // device instructions, uploads and downloads
   bool has_hostdata = false;
+  bool reads_download = false;  // looks at a value that an earlier span copied to the host
+  bool collects = false;        // the last span with device work: it also copies the function's results out
+  std::vector<int> steady_host;  // instructions of pass 1 that a steady run fires
+  CopyJobs uploads;              // this run's uploads, in program order
+  CopyJobs captured_uploads;     // what the copy node of `exec` was last told
+  cudaGraphNode_t upload_node = nullptr;
+  cudaGraph_t graph = nullptr;   // kept: `upload_node` belongs to it
   cudaGraphExec_t exec = nullptr;
   uint64_t exec_key = 0, last_key = 0;
   bool have_last = false, capture_failed = false;
@@ -97,6 +111,12 @@ struct cgtbInterp {
   bool host_dirty = false;              // a host data instruction of this run produced a new value
   bool prev_run_ok = false;
   uint64_t args_read_in_place = ~0ull;  // arguments whose device buffer a captured instruction reads directly
+  std::vector<char> downloaded;         // locations that a device->host copy writes
+  char* out_stage = nullptr;            // pinned block that holds the device results of the last run
+  long out_stage_cap = 0;
+  std::vector<void*> out_host;          // per result: its bytes in host memory, or null (not an array on the device)
+  std::vector<long> out_offset;
+  std::vector<cgtArray*> out_array;     // the array that was copied to out_host
   long last_host_ns = 0;                // host time of the last run up to the final wait for the stream
   long steady_runs = 0;
 };
@@ -116,7 +136,10 @@ CGTB_API cgtbGraph* cgtb_graph_new(long n_args, long n_locs) {
 }
 CGTB_API void cgtb_graph_free(cgtbGraph* g) {
   if (!g) return;
-  for (auto& in : g->instrs) free_scratch_owner(&in.scratch);
+  for (auto& in : g->instrs) {
+    free_scratch_owner(&in.scratch);
+    if (in.stage) cgtb_free(cgtbCPU, in.stage);
+  }
   delete g;
 }
 
@@ -198,9 +221,15 @@ CGTB_API int cgtb_graph_add_return_byval(cgtbGraph* g, const char* repr, int n, 
 // Cut the instruction list into spans at every barrier instruction. A fire-once barrier (a constant's
 // transport) that has already fired no longer separates its neighbours, so after the first run the
 // whole step usually collapses into one span per real transfer.
+static void drop_exec(Span& s) {
+  if (s.exec) cudaGraphExecDestroy(s.exec);
+  if (s.graph) cudaGraphDestroy(s.graph);
+  s.exec = nullptr;
+  s.graph = nullptr;
+  s.upload_node = nullptr;
+}
 static void build_spans(cgtbInterp* it) {
-  for (auto& s : it->spans)
-    if (s.exec) cudaGraphExecDestroy(s.exec);
+  for (auto& s : it->spans) drop_exec(s);
   it->spans.clear();
   auto& instrs = it->g->instrs;
   int n = (int)instrs.size();
@@ -208,24 +237,53 @@ static void build_spans(cgtbInterp* it) {
     Instr& in = instrs[(size_t)k];
     return in.klass == kBarrier && !((in.flags & CGTB_INSTR_ONCE) && in.fired);
   };
+  auto reads_downloaded = [&](const Instr& in) {
+    for (auto& r : in.reads)
+      if (it->downloaded[(size_t)r.idx]) return true;
+    return false;
+  };
+  it->downloaded.assign((size_t)it->g->n_locs, 0);
   int i = 0;
   while (i < n) {
     Span s;
     s.begin = i;
+    s.uploads.n = s.captured_uploads.n = 0;
     if (is_barrier(i)) {
       s.barrier = true;
       s.end = i + 1;
     } else {
-      int j = i;
+      int j = i, n_uploads = 0, n_downloads = 0;
+      std::vector<char> fresh((size_t)it->g->n_locs, 0);  // copied to the host by this span
       while (j < n && !is_barrier(j)) {
-        if (instrs[(size_t)j].klass == kDevice) s.n_device++;
-        if (instrs[(size_t)j].klass == kHostData) s.has_hostdata = true;
+        Instr& in = instrs[(size_t)j];
+        if (n_downloads) {
+          // only bookkeeping and further downloads may follow a download in its span
+          bool cut = in.klass != kMeta && in.klass != kDownload;
+          for (auto& r : in.reads) cut = cut || fresh[(size_t)r.idx];
+          if (cut || (in.klass == kDownload && n_downloads == kMaxCopyJobs)) break;
+        }
+        if (in.klass == kUpload && n_uploads == kMaxCopyJobs) break;
+        if (in.klass == kDownload) {
+          ++n_downloads;
+          fresh[(size_t)in.write.idx] = 1;
+        }
+        if (in.klass == kUpload) ++n_uploads;
+        if (in.klass == kDevice || in.klass == kUpload || in.klass == kDownload) s.n_device++;
+        if (in.klass == kHostData) s.has_hostdata = true;
+        if (in.klass != kDevice && reads_downloaded(in)) s.reads_download = true;
+        if (in.klass == kHostData || in.klass == kUpload || (in.klass == kMeta && in.arg_view)) s.steady_host.push_back(j);
         ++j;
       }
+      for (size_t l = 0; l < fresh.size(); ++l) it->downloaded[l] |= fresh[l];
       s.end = j;
     }
     it->spans.push_back(s);
     i = s.end;
+  }
+  // results are collected by the last span that has device work, unless a non-capturable instruction comes later
+  for (size_t k = it->spans.size(); k-- > 0;) {
+    if (it->spans[k].barrier) break;
+    if (it->spans[k].n_device > 0) { it->spans[k].collects = true; break; }
   }
 }
 
@@ -241,7 +299,11 @@ CGTB_API cgtbInterp* cgtb_interp_new(cgtbGraph* g, int n_out, const long* out_lo
   }
   bool any_device = false;
   for (auto& in : g->instrs) {
+    const bool plain_copy = (in.flags & CGTB_INSTR_TRANSPORT) && !(in.flags & (CGTB_INSTR_NOCAPTURE | CGTB_INSTR_ONCE)) &&
+                            in.kind == kReturnByRef && in.reads.size() == 1 && !(flags & CGTB_INTERP_PROFILE);
     if (in.kind == kLoadArgument || in.kind == kAlloc || in.kind == kBuildTup) in.klass = kMeta;
+    else if (plain_copy && in.reads[0].dev == cgtbCPU && in.write.dev == cgtbGPU) in.klass = kUpload;
+    else if (plain_copy && in.reads[0].dev == cgtbGPU && in.write.dev == cgtbCPU) in.klass = kDownload;
     else if (in.flags & (CGTB_INSTR_TRANSPORT | CGTB_INSTR_NOCAPTURE)) in.klass = kBarrier;
     else if (in.flags & CGTB_INSTR_QUICK) in.klass = kMeta;
     else if (in.write.dev == cgtbGPU) in.klass = (in.kind == kReturnByRef) ? kDevice : kBarrier;
@@ -280,8 +342,8 @@ CGTB_API cgtbInterp* cgtb_interp_new(cgtbGraph* g, int n_out, const long* out_lo
 CGTB_API void cgtb_interp_free(cgtbInterp* it) {
   if (!it) return;
   if (rt().ready) cudaStreamSynchronize(rt().stream);
-  for (auto& s : it->spans)
-    if (s.exec) cudaGraphExecDestroy(s.exec);
+  for (auto& s : it->spans) drop_exec(s);
+  if (it->out_stage) cgtb_free(cgtbCPU, it->out_stage);
   delete it;
 }
 
@@ -371,12 +433,15 @@ static uint64_t key_of_object(uint64_t h, cgtObject* o, int dev) {
   if (!o) return mix(h, 0);
   if (o->kind() == cgtObject::ArrayKind) {
     cgtArray* a = (cgtArray*)o;
-    h = mix(h, (uint64_t)(uintptr_t)a->data());
+    // a small host operand counts by its bytes alone: kernels receive its value at launch, and the object that holds it
+    // (a Size, a host scalar) may be a new one on every run
+    const bool by_value = a->devtype() == cgtCPU && a->nbytes() <= 64 && a->data();
+    if (!by_value) h = mix(h, (uint64_t)(uintptr_t)a->data());
     // a captured graph bakes shape-derived launch parameters into its nodes, and the pool can hand the same block
     // to a differently shaped array of equal size: the extents and the dtype are part of the key
     h = mix(h, ((uint64_t)a->ndim() << 8) | (uint64_t)a->dtype());
     for (int d = 0; d < a->ndim(); ++d) h = mix(h, (uint64_t)a->shape()[d]);
-    if (a->devtype() == cgtCPU && a->nbytes() <= 64 && a->data()) {  // small host operand read at launch time
+    if (by_value) {
       uint64_t buf[8] = {0};
       memcpy(buf, a->data(), (size_t)a->nbytes());
       for (int i = 0; i < 8; ++i) h = mix(h, buf[i]);
@@ -387,13 +452,24 @@ static uint64_t key_of_object(uint64_t h, cgtObject* o, int dev) {
   }
   return h;
 }
+static void* array_data(cgtObject* o) { return o && o->kind() == cgtObject::ArrayKind ? ((cgtArray*)o)->data() : nullptr; }
 static uint64_t span_key(cgtbInterp* it, const Span& s) {
   uint64_t h = 1469598103934665603ull;
   for (int i = s.begin; i < s.end; ++i) {
     Instr& in = it->g->instrs[(size_t)i];
+    // an upload's source is not part of the key: its copy node is told the new address before each launch
+    if (in.klass == kUpload) h = key_of_object(h, get(it, in.write), in.write.dev);
+    if (in.klass == kDownload) h = mix(key_of_object(h, get(it, in.reads[0]), in.reads[0].dev), (uint64_t)(uintptr_t)array_data(get(it, in.write)));
     if (in.klass != kDevice) continue;
     for (auto& r : in.reads) h = key_of_object(h, get(it, r), r.dev);
     h = key_of_object(h, get(it, in.write), in.write.dev);
+  }
+  if (s.collects) {
+    h = mix(h, (uint64_t)(uintptr_t)it->out_stage);
+    for (auto& o : it->outs) {
+      cgtObject* obj = get(it, o);
+      if (obj && obj->kind() == cgtObject::ArrayKind && ((cgtArray*)obj)->devtype() == cgtGPU) h = key_of_object(h, obj, cgtbGPU);
+    }
   }
   return h;
 }
@@ -554,6 +630,163 @@ static int fire_span_multistream(cgtbInterp* it, Span& s, cudaStream_t origin) {
   return rc;
 }
 
+// ------------------------------------------------------------------------------------------------
+// Copies between host and device: uploads at a span's start, downloads and results at its end
+// ------------------------------------------------------------------------------------------------
+// Host part of an upload (pass 1, in program order): what the copy kernel will read is put in place, or a large host
+// array is sent through the copy engine at once.
+static int stage_upload(cgtbInterp* it, Span& s, Instr& in) {
+  cgtObject *src_o = get(it, in.reads[0]), *dst_o = get(it, in.write);
+  if (!src_o || !dst_o) return fail("%s: operand was never produced", in.repr.c_str());
+  if (src_o->kind() != cgtObject::ArrayKind || dst_o->kind() != cgtObject::ArrayKind) return fire(it, in);  // tuples: member by member
+  cgtArray *src = (cgtArray*)src_o, *dst = (cgtArray*)dst_o;
+  const long nbytes = src->nbytes();
+  if (src->size() != dst->size() || src->dtype() != dst->dtype()) return fail("%s: cgt_copy_array: size or dtype mismatch", in.repr.c_str());
+  if (nbytes == 0) return 0;
+  const void* from = src->data();
+  if (src->devtype() == cgtCPU) {
+    const bool pinned = host_block_is_pinned(from);
+    if (nbytes > kKernelCopyBytes) {
+      if (!pinned) return upload_pageable(dst->data(), from, (size_t)nbytes);
+      CGTB_CUDA_TRY(cudaMemcpyAsync(dst->data(), from, (size_t)nbytes, cudaMemcpyHostToDevice, rt().stream));
+      return 0;
+    }
+    if (!pinned) {
+      if (in.stage_cap < nbytes) {
+        if (in.stage) cgtb_free(cgtbCPU, in.stage);
+        in.stage = cgtb_alloc(cgtbCPU, nbytes);
+        in.stage_cap = in.stage ? nbytes : 0;
+        if (!in.stage) return 1;
+      }
+      stage_for_kernel(in.stage, from, (size_t)nbytes);
+      from = in.stage;
+    }
+  }
+  s.uploads.job[s.uploads.n++] = CopyJob{from, dst->data(), nbytes};
+  return 0;
+}
+
+static void add_copy_out(CopyJobs& jobs, const void* src, void* dst, long nbytes, int* rc) {
+  if (nbytes == 0 || *rc) return;
+  if (nbytes > kKernelCopyBytes) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, (size_t)nbytes, cudaMemcpyDeviceToHost, rt().stream);
+    if (e != cudaSuccess) *rc = fail("copy to the host failed: %s", cudaGetErrorString(e));
+    return;
+  }
+  if (jobs.n == kMaxCopyJobs) {
+    *rc = launch_copy_jobs(jobs);
+    jobs.n = 0;
+  }
+  jobs.job[jobs.n++] = CopyJob{src, dst, nbytes};
+}
+// Place of every device result in the pinned result block (grown here, outside captures).
+static int place_outputs(cgtbInterp* it) {
+  long total = 0;
+  it->out_offset.assign(it->outs.size(), -1);
+  it->out_array.assign(it->outs.size(), nullptr);
+  for (size_t i = 0; i < it->outs.size(); ++i) {
+    cgtObject* o = get(it, it->outs[i]);
+    if (!o || o->kind() != cgtObject::ArrayKind || ((cgtArray*)o)->devtype() != cgtGPU) continue;
+    it->out_offset[i] = total;
+    it->out_array[i] = (cgtArray*)o;
+    total += (((cgtArray*)o)->nbytes() + 63) & ~63L;
+  }
+  if (total > it->out_stage_cap) {
+    if (it->out_stage) cgtb_free(cgtbCPU, it->out_stage);
+    it->out_stage = (char*)cgtb_alloc(cgtbCPU, total);
+    it->out_stage_cap = it->out_stage ? total : 0;
+    if (!it->out_stage) return 1;
+  }
+  return 0;
+}
+static void add_outputs(cgtbInterp* it, CopyJobs& jobs, int* rc) {
+  for (size_t i = 0; i < it->outs.size(); ++i) {
+    it->out_host[i] = nullptr;
+    if (it->out_offset[i] < 0) continue;
+    cgtArray* a = it->out_array[i];
+    it->out_host[i] = it->out_stage + it->out_offset[i];
+    add_copy_out(jobs, a->data(), it->out_host[i], a->nbytes(), rc);
+  }
+}
+// Copies that end the span: its downloads, and the function's results if it is the last one.
+static int issue_copies_out(cgtbInterp* it, Span& s) {
+  auto& instrs = it->g->instrs;
+  CopyJobs jobs;
+  jobs.n = 0;
+  int rc = 0;
+  for (int i = s.begin; i < s.end && !rc; ++i) {
+    Instr& in = instrs[(size_t)i];
+    if (in.klass != kDownload) continue;
+    cgtObject *src = get(it, in.reads[0]), *dst = get(it, in.write);
+    if (!src || !dst) return fail("%s: operand was never produced", in.repr.c_str());
+    if (src->kind() != cgtObject::ArrayKind || dst->kind() != cgtObject::ArrayKind || ((cgtArray*)src)->devtype() != cgtGPU ||
+        !host_block_is_pinned(((cgtArray*)dst)->data())) {
+      rc = fire(it, in);
+      continue;
+    }
+    cgtArray *a = (cgtArray*)src, *b = (cgtArray*)dst;
+    if (a->size() != b->size() || a->dtype() != b->dtype()) return fail("%s: cgt_copy_array: size or dtype mismatch", in.repr.c_str());
+    add_copy_out(jobs, a->data(), b->data(), a->nbytes(), &rc);
+  }
+  if (s.collects && !rc) add_outputs(it, jobs, &rc);
+  return rc ? rc : launch_copy_jobs(jobs);
+}
+static int issue_device(cgtbInterp* it, Span& s, bool profile, bool multistream) {
+  auto& instrs = it->g->instrs;
+  if (launch_copy_jobs(s.uploads)) return 1;
+  if (multistream) {
+    if (fire_span_multistream(it, s, rt().stream)) return 1;
+  } else {
+    for (int i = s.begin; i < s.end; ++i) {
+      Instr& in = instrs[(size_t)i];
+      if (in.klass != kDevice) continue;
+      if ((in.flags & CGTB_INSTR_ONCE) && in.fired) continue;
+      const int rc = profile ? fire_profiled(it, in) : fire(it, in);
+      if (rc) return rc;
+    }
+  }
+  return issue_copies_out(it, s);
+}
+static void mark_device_fired(cgtbInterp* it, Span& s) {
+  for (int i = s.begin; i < s.end; ++i)
+    if (it->g->instrs[(size_t)i].klass == kDevice) it->g->instrs[(size_t)i].fired = true;
+}
+// The graph's first node is the copy kernel (if the span uploads anything): remember it for update_uploads.
+static void find_upload_node(Span& s) {
+  s.upload_node = nullptr;
+  if (!s.uploads.n) return;
+  size_t n = 0;
+  if (cudaGraphGetRootNodes(s.graph, nullptr, &n) != cudaSuccess || n != 1) return;
+  cudaGraphNode_t node;
+  cudaKernelNodeParams p;
+  if (cudaGraphGetRootNodes(s.graph, &node, &n) == cudaSuccess && cudaGraphKernelNodeGetParams(node, &p) == cudaSuccess && p.func == copy_jobs_function())
+    s.upload_node = node;
+}
+// Before a replay: tell the copy node where this run's arguments are, if they moved. false: the graph cannot be used.
+static bool update_uploads(Span& s) {
+  const CopyJobs &a = s.uploads, &b = s.captured_uploads;
+  if (a.n == b.n && memcmp(a.job, b.job, sizeof(CopyJob) * (size_t)a.n) == 0) return true;
+  if (a.n != b.n || !s.upload_node) return false;
+  unsigned gx, gy, block;
+  copy_jobs_launch_dims(s.uploads, &gx, &gy, &block);
+  cudaKernelNodeParams p = {};
+  void* args[1] = {&s.uploads};
+  p.func = const_cast<void*>(copy_jobs_function());
+  p.gridDim = dim3(gx, gy);
+  p.blockDim = dim3(block);
+  p.kernelParams = args;
+  if (cudaGraphExecKernelNodeSetParams(s.exec, s.upload_node, &p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  s.captured_uploads = s.uploads;
+  return true;
+}
+// a replay leaves the results where the captured run put them
+static void outputs_of_replay(cgtbInterp* it) {
+  for (size_t i = 0; i < it->outs.size(); ++i) it->out_host[i] = it->out_offset[i] < 0 ? nullptr : it->out_stage + it->out_offset[i];
+}
+
 static int run_span(cgtbInterp* it, Span& s) {
   auto& instrs = it->g->instrs;
   const bool profile = (it->flags & CGTB_INTERP_PROFILE) && rt().ready;
@@ -571,18 +804,26 @@ static int run_span(cgtbInterp* it, Span& s) {
     if (is_transport && in.write.dev == cgtbCPU) it->host_pending = true;
     return 0;
   }
-  if (s.has_hostdata && it->host_pending) {
+  if ((s.has_hostdata || s.reads_download) && it->host_pending) {
     CGTB_CUDA_TRY(cudaStreamSynchronize(rt().stream));
     it->host_pending = false;
   }
-  // pass 1: host bookkeeping and host scalar arithmetic, in program order
-  for (int i = s.begin; i < s.end; ++i) {
+  s.uploads.n = 0;
+  // pass 1: host bookkeeping and host scalar arithmetic, in program order. A steady run skips bookkeeping whose result
+  // the storage already holds.
+  const bool steady_list = it->steady && !it->host_dirty;
+  const int n_pass1 = steady_list ? (int)s.steady_host.size() : s.end - s.begin;
+  for (int q = 0; q < n_pass1; ++q) {
+    const int i = steady_list && !it->host_dirty ? s.steady_host[(size_t)q] : (steady_list ? -1 : s.begin + q);
+    if (i < 0) break;  // a host value changed within this span: the rest is walked in full below
     Instr& in = instrs[(size_t)i];
-    if (in.klass == kDevice) continue;
+    if (in.klass == kDevice || in.klass == kDownload) continue;
     if ((in.flags & CGTB_INSTR_ONCE) && in.fired) continue;
-    const bool fast = it->steady && !it->host_dirty;
-    if (fast && in.klass == kMeta && !in.arg_view) continue;  // the storage already holds its result
-    if (fast && in.klass == kHostData) {
+    if (in.klass == kUpload) {
+      if (stage_upload(it, s, in)) return 1;
+      continue;
+    }
+    if (steady_list && in.klass == kHostData) {
       // did this instruction produce the value it produced in the run before? (small results only: a large one
       // counts as new)
       unsigned char before[64];
@@ -597,28 +838,38 @@ static int run_span(cgtbInterp* it, Span& s) {
       }
       if (fire(it, in)) return 1;
       cgtObject* w2 = get(it, in.write);
-      if (!small || w2 != w || memcmp(before, ((cgtArray*)w2)->data(), nb) != 0) it->host_dirty = true;
+      if (!small || w2 != w || memcmp(before, ((cgtArray*)w2)->data(), nb) != 0) {
+        it->host_dirty = true;
+        in.fired = true;
+        // everything after this instruction is walked in full
+        for (int k = i + 1; k < s.end; ++k) {
+          Instr& rest = instrs[(size_t)k];
+          if (rest.klass == kDevice || rest.klass == kDownload) continue;
+          if ((rest.flags & CGTB_INSTR_ONCE) && rest.fired) continue;
+          if (rest.klass == kUpload ? stage_upload(it, s, rest) : fire(it, rest)) return 1;
+          rest.fired = true;
+        }
+      }
       in.fired = true;
       continue;
     }
     if (fire(it, in)) return 1;
     in.fired = true;
   }
+  // on every run, steady ones too: bookkeeping on arguments makes a new view object of the same bytes each time
+  if (s.collects && place_outputs(it)) return 1;
   if (s.n_device == 0) return 0;
+  for (int i = s.begin; i < s.end && !it->host_pending; ++i) it->host_pending = instrs[(size_t)i].klass == kDownload;
   // pass 2: device instructions, replayed from a CUDA graph when the span is in steady state
   bool use_graphs = (it->flags & CGTB_INTERP_CUDA_GRAPHS) && !profile && !s.capture_failed && s.n_device >= 2;
-  if (use_graphs && it->steady && !it->host_dirty && s.exec && s.have_last && s.exec_key == s.last_key) {
-    // nothing that the key covers can have changed since the run before, which launched this graph
-    CGTB_CUDA_TRY(cudaGraphLaunch(s.exec, rt().stream));
-    it->last_graph_launches += 1;
-    it->last_launches += s.graph_kernels;
-    return 0;
-  }
-  uint64_t key = use_graphs ? span_key(it, s) : 0;
-  if (use_graphs && s.exec && s.exec_key == key) {
+  const bool unchanged = it->steady && !it->host_dirty && s.exec && s.have_last && s.exec_key == s.last_key;
+  uint64_t key = use_graphs && !unchanged ? span_key(it, s) : s.last_key;
+  // `unchanged`: nothing that the key covers can have changed since the run before, which launched this graph
+  if (use_graphs && s.exec && s.exec_key == key && update_uploads(s)) {
     s.last_key = key;
     s.have_last = true;
     CGTB_CUDA_TRY(cudaGraphLaunch(s.exec, rt().stream));
+    if (s.collects) outputs_of_replay(it);
     it->last_graph_launches += 1;
     it->last_launches += s.graph_kernels;
     return 0;
@@ -627,39 +878,31 @@ static int run_span(cgtbInterp* it, Span& s) {
   s.last_key = key;
   s.have_last = true;
   if (capture) {
-    if (s.exec) { cudaGraphExecDestroy(s.exec); s.exec = nullptr; }
+    drop_exec(s);
     long launches0 = g_kernel_launches.load();
     cudaError_t e = cudaStreamBeginCapture(rt().stream, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
       set_capturing(true);
-      int rc = 0;
-      if (graph_streams() > 1) {
-        rc = fire_span_multistream(it, s, rt().stream);
-      } else {
-        for (int i = s.begin; i < s.end && !rc; ++i) {
-          Instr& in = instrs[(size_t)i];
-          if (in.klass != kDevice) continue;
-          if ((in.flags & CGTB_INSTR_ONCE) && in.fired) continue;
-          rc = fire(it, in);
-        }
-      }
+      int rc = issue_device(it, s, false, graph_streams() > 1);
       set_capturing(false);
       cudaGraph_t graph = nullptr;
       e = cudaStreamEndCapture(rt().stream, &graph);
       if (rc == 0 && e == cudaSuccess && graph) {
         e = cudaGraphInstantiate(&s.exec, graph, 0);
-        cudaGraphDestroy(graph);
         if (e == cudaSuccess) {
+          s.graph = graph;
+          find_upload_node(s);
+          s.captured_uploads = s.uploads;
           s.exec_key = key;   // == s.last_key
           s.graph_kernels = g_kernel_launches.load() - launches0;
           it->captured += 1;
-          for (int i = s.begin; i < s.end; ++i)
-            if (instrs[(size_t)i].klass == kDevice) instrs[(size_t)i].fired = true;
+          mark_device_fired(it, s);
           CGTB_CUDA_TRY(cudaGraphLaunch(s.exec, rt().stream));
           it->last_graph_launches += 1;
           it->last_launches += s.graph_kernels;
           return 0;
         }
+        cudaGraphDestroy(graph);
         s.exec = nullptr;
       } else if (graph) {
         cudaGraphDestroy(graph);
@@ -670,16 +913,10 @@ static int run_span(cgtbInterp* it, Span& s) {
     cgtb_clear_error();
     s.capture_failed = true;
   }
-  for (int i = s.begin; i < s.end; ++i) {
-    Instr& in = instrs[(size_t)i];
-    if (in.klass != kDevice) continue;
-    if ((in.flags & CGTB_INSTR_ONCE) && in.fired) continue;
-    long l0 = g_kernel_launches.load();
-    int rc = profile ? fire_profiled(it, in) : fire(it, in);
-    if (rc) return rc;
-    in.fired = true;
-    it->last_launches += g_kernel_launches.load() - l0;
-  }
+  long l0 = g_kernel_launches.load();
+  if (issue_device(it, s, profile, false)) return 1;
+  mark_device_fired(it, s);
+  it->last_launches += g_kernel_launches.load() - l0;
   return 0;
 }
 
@@ -739,14 +976,23 @@ CGTB_API int cgtb_interp_run(cgtbInterp* it, cgtbObject* args_obj, cgtbObject** 
   long last_queueing = -1;
   for (size_t i = 0; i < it->spans.size(); ++i)
     if (it->spans[i].barrier || it->spans[i].n_device > 0) last_queueing = (long)i;
-  bool hooked = false;
+  bool hooked = false, collected = false;
+  it->out_host.assign(it->outs.size(), nullptr);
   for (size_t i = 0; i < it->spans.size(); ++i) {
     rc = run_span(it, it->spans[i]);
     if (rc) break;
+    collected = collected || it->spans[i].collects;
     if ((long)i == last_queueing && it->before_sync) {
       it->before_sync(it->before_sync_ctx);
       hooked = true;
     }
+  }
+  if (!rc && !collected && rt().ready) {
+    CopyJobs jobs;
+    jobs.n = 0;
+    rc = place_outputs(it);
+    if (!rc) add_outputs(it, jobs, &rc);
+    if (!rc) rc = launch_copy_jobs(jobs);
   }
   it->args = nullptr;
   if (!rc && !hooked && it->before_sync) it->before_sync(it->before_sync_ctx);
@@ -764,9 +1010,17 @@ CGTB_API int cgtb_interp_run(cgtbInterp* it, cgtbObject* args_obj, cgtbObject** 
   if (rc) return rc;
   cgtTuple* o = new cgtTuple((int)it->outs.size());
   o->Retain();
-  for (size_t i = 0; i < it->outs.size(); ++i) o->setitem((int)i, get(it, it->outs[i]));
+  for (size_t i = 0; i < it->outs.size(); ++i) {
+    o->setitem((int)i, get(it, it->outs[i]));
+    // an object that bookkeeping replaced after the results were copied is read back by the caller
+    if (it->out_host[i] && get(it, it->outs[i]) != it->out_array[i]) it->out_host[i] = nullptr;
+  }
   *out = (cgtbObject*)o;
   return 0;
+}
+
+CGTB_API const void* cgtb_interp_output_host(cgtbInterp* it, int i) {
+  return it && i >= 0 && (size_t)i < it->out_host.size() ? it->out_host[(size_t)i] : nullptr;
 }
 
 CGTB_API int cgtb_interp_set_before_sync(cgtbInterp* it, void (*fn)(void*), void* ctx) {

@@ -4,6 +4,7 @@
 // Replaces src/cgt_common.cpp of the reference (cudaMalloc / cudaFree / synchronous cudaMemcpy per
 // array) with pooled, stream-ordered equivalents.
 #include "runtime.h"
+#include "host_copy.h"
 #include <cstdarg>
 #include <cstring>
 #include <map>
@@ -116,7 +117,9 @@ struct HostSlabs {
   std::mutex mu;
   static constexpr size_t kSlab = 1 << 20, kMaxSmall = 4096;
   char* cur = nullptr;
+  bool cur_pinned = false;
   size_t used = kSlab;
+  std::vector<char*> unpinned;  // slabs from before a GPU was bound: their blocks are not handed out again after that
   std::map<size_t, std::vector<void*>> free_lists;
   std::unordered_map<void*, size_t> live;
   static size_t cls(size_t n) { size_t c = 64; while (c < n) c *= 2; return c; }
@@ -127,11 +130,17 @@ struct HostSlabs {
     void* p;
     if (!fl.empty()) { p = fl.back(); fl.pop_back(); }
     else {
-      if (used + c > kSlab) {
+      if (used + c > kSlab || (g_rt.ready && !cur_pinned)) {
         void* s = nullptr;
-        cudaError_t e = g_rt.ready ? cudaHostAlloc(&s, kSlab, cudaHostAllocDefault) : cudaErrorInitializationError;
-        if (e != cudaSuccess) { s = aligned_alloc(64, kSlab); }  // no GPU: plain host memory
+        if (g_rt.ready) {
+          cudaError_t e = cudaHostAlloc(&s, kSlab, cudaHostAllocDefault);
+          if (e != cudaSuccess) { fail("cudaHostAlloc failed: %s", cudaGetErrorString(e)); return nullptr; }
+        } else {
+          s = aligned_alloc(64, kSlab);  // no GPU: plain host memory
+          unpinned.push_back((char*)s);
+        }
         cur = (char*)s;
+        cur_pinned = g_rt.ready;
         used = 0;
       }
       p = cur + used;
@@ -144,12 +153,31 @@ struct HostSlabs {
     std::lock_guard<std::mutex> lk(mu);
     auto it = live.find(p);
     if (it == live.end()) return false;
-    free_lists[it->second].push_back(p);
+    if (!g_rt.ready || pinned(p)) free_lists[it->second].push_back(p);
     live.erase(it);
     return true;
   }
+  bool pinned(const void* p) const {
+    for (char* s : unpinned)
+      if ((const char*)p >= s && (const char*)p < s + kSlab) return false;
+    return true;
+  }
+  void runtime_bound() {  // only pinned blocks from here on
+    std::lock_guard<std::mutex> lk(mu);
+    free_lists.clear();
+  }
 };
 static HostSlabs g_slabs;
+
+bool host_block_is_pinned(const void* p) {
+  if (!g_rt.ready) return false;
+  {
+    std::lock_guard<std::mutex> lk(g_slabs.mu);
+    if (g_slabs.live.count(const_cast<void*>(p))) return g_slabs.pinned(p);
+  }
+  std::lock_guard<std::mutex> lk(g_host_pool.mu);
+  return g_host_pool.live.count(const_cast<void*>(p)) != 0;
+}
 
 static thread_local bool t_capturing = false;
 void set_capturing(bool on) { t_capturing = on; }
@@ -217,6 +245,7 @@ CGTB_API int cgtb_init(int device) {
   g_rt.device = device;
   g_rt.sm_count = prop.multiProcessorCount;
   g_host_pool.pinned_host = true;
+  g_slabs.runtime_bound();
   g_rt.ready = true;
   return 0;
 }
@@ -242,6 +271,7 @@ CGTB_API int cgtb_pool_trim(void) {
   if (!require_runtime("cgtb_pool_trim")) return 1;
   cudaStreamSynchronize(g_rt.stream);
   g_dev_pool.trim();
+  trim_staging();
   return 0;
 }
 CGTB_API long cgtb_kernel_launches(void) { return g_kernel_launches.load(); }

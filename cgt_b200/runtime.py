@@ -73,7 +73,8 @@ def _declare(lib):
         "cgtb_graph_add_return_byval": (ci, [vp, ctypes.c_char_p, ci, c_long_p, c_int_p, cl, ci, vp, vp, ci]),
         "cgtb_interp_new": (vp, [vp, ci, c_long_p, ci]), "cgtb_interp_free": (None, [vp]),
         "cgtb_interp_set_before_sync": (ci, [vp, vp, vp]),
-        "cgtb_interp_run": (ci, [vp, vp, ctypes.POINTER(vp)]), "cgtb_interp_stats": (ci, [vp, c_long_p, ci]), "cgtb_state_version_bump": (None, []),
+        "cgtb_interp_run": (ci, [vp, vp, ctypes.POINTER(vp)]), "cgtb_interp_output_host": (vp, [vp, ci]),
+        "cgtb_host_copy": (None, [vp, vp, cl]), "cgtb_interp_stats": (ci, [vp, c_long_p, ci]), "cgtb_state_version_bump": (None, []),
         "cgtb_interp_profile": (ci, [vp, ctypes.POINTER(cd), c_long_p, ci]),
         "cgtb_interp_instr_repr": (ctypes.c_char_p, [vp, ci]),
         "cgtb_apply_byref": (ci, [vp, vp, ci, ctypes.POINTER(vp), vp]),
@@ -399,6 +400,23 @@ def apply_byref(fptr, cldata, inputs, output):
 # ------------------------------------------------------------------------------------------------
 # interpreter wrapper (src/cycgt.pyx:404-434)
 # ------------------------------------------------------------------------------------------------
+_bridge_module = None
+
+
+def _bridge():
+    """The native call path (csrc/pybridge.cpp); built together with the library."""
+    global _bridge_module
+    if _bridge_module is None:
+        lib()
+        try:
+            from . import _pybridge
+        except ImportError as e:
+            raise BackendError("cgt_b200/_pybridge.so is missing or was built for another Python (%s): build it with "
+                               "`python -m cgt_b200.build`" % e)
+        _bridge_module = _pybridge
+    return _bridge_module
+
+
 _BYREF_T = ctypes.CFUNCTYPE(None, ctypes.c_void_p, ctypes.POINTER(ctypes.c_void_p), ctypes.c_void_p)
 _BYVAL_T = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_void_p, ctypes.POINTER(ctypes.c_void_p))
 
@@ -427,9 +445,17 @@ def _obj_view(h):
 class InterpreterWrapper(object):
     """Builds the native execution graph from the Python one and runs it."""
 
-    def __init__(self, pyeg, input_types, output_locs, flags):
+    def __init__(self, pyeg, input_types, output_locs, flags, tuple_outputs=False):
         from . import compilation
         L = lib()
+        self._pf_request = None   # arguments announced by prefetch() and not yet uploaded
+        self._pf = {}             # slot -> uploads that no call has used yet
+        self._pf_error = None
+        # (type number, rank) per argument for the native call path; None: some argument or result is a tuple
+        self._fast_types = None
+        if not tuple_outputs and len(input_types) <= 32 and all(hasattr(t, "ndim") and t.dtype in DTYPE_NUM for t in input_types):
+            self._fast_types = bytes(b for t in input_types for b in (DTYPE_NUM[t.dtype], t.ndim))
+            self._fast_run = _bridge().run
         self.storage = []  # keeps callables, closures and trampolines alive
         self.input_types = input_types
         self.n_instrs = len(pyeg.instrs)
@@ -460,6 +486,7 @@ class InterpreterWrapper(object):
         self.interp = L.cgtb_interp_new(self.graph, len(output_locs), olocs, flags)
         if not self.interp:
             raise BackendError(last_error())
+        self._interp_addr = ctypes.cast(self.interp, ctypes.c_void_p).value
 
     def _marshal(self, callable_, instr):
         from . import compilation
@@ -524,7 +551,7 @@ class InterpreterWrapper(object):
         L = lib()
         pyargs, self._pf_request = self._pf_request, None
         if not hasattr(self, "_pf_bufs"):
-            self._pf_bufs, self._pf_slot, self._pf = ({}, {}), 0, {}
+            self._pf_bufs, self._pf_slot = ({}, {}), 0
         self._pf_slot ^= 1
         slot, bufs = self._pf_slot, self._pf_bufs[self._pf_slot]
         check(L.cgtb_prefetch_begin(slot), "prefetch")
@@ -544,14 +571,30 @@ class InterpreterWrapper(object):
         self._pf[slot] = staged  # replaces an unconsumed upload that used this slot
 
     def __call__(self, *pyargs):
+        if self._fast_types is not None and not self._pf and self._pf_request is None:
+            out = self._fast_run(self._interp_addr, self._fast_types, pyargs, ArrayWrapper)
+            if out is not NotImplemented:
+                if self._pending_release:
+                    self._release_pending()
+                if type(out) is int:
+                    check(out, "running compiled function")
+                return out
+        return self._call_general(pyargs)
+
+    def _release_pending(self):
+        for h in self._pending_release:
+            lib().cgtb_release(h)
+        del self._pending_release[:]
+
+    def _call_general(self, pyargs):
         from . import core
         L = lib()
         assert len(pyargs) == len(self.input_types), "expected %d arguments, got %d" % (len(self.input_types), len(pyargs))
-        request = getattr(self, "_pf_request", None)
+        request = self._pf_request
         if request is not None and any(r is a for (r, a) in zip(request, pyargs) if not isinstance(a, (ArrayWrapper, tuple))):
             self._pf_issue()  # announced for this very call: upload now
         used_slot = None
-        for (slot, staged) in list(getattr(self, "_pf", {}).items()):
+        for (slot, staged) in list(self._pf.items()):
             hits = [i for (i, (arg, _a, _w)) in staged.items() if pyargs[i] is arg]
             if hits:
                 pyargs = list(pyargs)
@@ -589,18 +632,27 @@ class InterpreterWrapper(object):
         L.cgtb_release(cargs)
         if used_slot is not None:
             L.cgtb_prefetch_release(used_slot)  # the slot's buffers are free once this step has run
-        for h in self._pending_release:
-            L.cgtb_release(h)
-        del self._pending_release[:]
+        self._release_pending()
         check(rc, "running compiled function")
         try:
-            err = getattr(self, "_pf_error", None)
+            err = self._pf_error
             if err is not None:
                 self._pf_error = None
                 raise err
-            return list(cgt2py_object(out.value))
+            return [self._output(i, L.cgtb_tuple_get(out, i)) for i in range(L.cgtb_tuple_len(out))]
         finally:
             L.cgtb_release(out)
+
+    def _output(self, i, h):
+        """Output i as a new numpy array: from the host copy that the run made of it, if there is one."""
+        L = lib()
+        src = L.cgtb_interp_output_host(self.interp, i)
+        if not src:
+            return cgt2py_object(h)
+        shp = L.cgtb_array_shape(h)
+        out = np.empty(tuple(shp[d] for d in range(L.cgtb_array_ndim(h))), NUM_DTYPE[L.cgtb_array_dtype(h)])
+        L.cgtb_host_copy(ctypes.c_void_p(out.ctypes.data), ctypes.c_void_p(src), out.nbytes)
+        return out
 
     def stats(self):
         vals = (ctypes.c_long * 8)()

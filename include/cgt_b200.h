@@ -118,6 +118,10 @@ void cgtb_interp_free(cgtbInterp* it);
 /* args: tuple of arrays (host or device). *out: new reference to a tuple of the output objects.
  * Returns after the runtime stream has been synchronised, so host outputs are readable. */
 int cgtb_interp_run(cgtbInterp* it, cgtbObject* args, cgtbObject** out);
+/* Bytes of output i of the last run in host memory, for an array that lives on the device: they were copied there with
+ * the run's device work and stay until the next run. NULL for other outputs (host arrays, tuples). */
+const void* cgtb_interp_output_host(cgtbInterp* it, int i);
+void cgtb_host_copy(void* dst, const void* src, long nbytes); /* memcpy, by several threads when it is large */
 /* counters: [0] runs, [1] kernels launched by instructions in the last run, [2] graph launches in the
  * last run, [3] segments captured so far, [4] kernels inside captured graphs, [5] device instructions in the graph,
  * [6] host nanoseconds of the last run up to its final wait for the stream, [7] steady runs so far (runs that
