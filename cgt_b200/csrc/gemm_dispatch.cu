@@ -1,9 +1,10 @@
 // Mul22 / BatchedMul22 entry points: choose between the tcgen05 tensor-core kernels (3xTF32 split
 // precision; TMA-fed for 16-byte-aligned operands, gemm_tma.cu, register-fed otherwise,
 // gemm_tcgen05.cu) and the fp32 FMA kernel (gemm_simt.cu).
-// Products with few outputs and a short K go to a one-thread-per-output kernel (gemm_simt.cu).
-// impl: 0 automatic, 1 FMA (tiled), 2 tensor cores (either feed), 3 register-fed only, 4 TMA-fed only,
-// 5 the small-product kernel only.
+// Smaller products go to the FMA tiles (gemm_tile.cu) or to a one-warp-per-output kernel (cgt_product.h).
+// impl: 0 automatic, 1 FMA (tiled, general), 2 tensor cores (either feed), 3 register-fed only, 4 TMA-fed only,
+// 5 the small-product kernel only, 6 the FMA tiles only.
+#include "products.h"
 #include "runtime.h"
 #include "tc_util.h"
 
@@ -17,27 +18,16 @@ int sgemm_tc(int tA, int tB, long P, long M, long N, long K, const float* A, lon
 int sgemm_tma(int tA, int tB, long P, long M, long N, long K, const float* A, long lda, long strideA, const float* B,
               long ldb, long strideB, float* C, long ldc, long strideC, const ConvEpilogue* ep = nullptr);
 
-int sgemm_small(int tA, int tB, long P, long M, long N, long K, const float* A, long lda, long strideA, const float* B,
-                long ldb, long strideB, float* C, long ldc, long strideC);
-int sgemm_tile16(int tA, int tB, long P, long M, long N, long K, const float* A, long lda, long strideA, const float* B,
-                 long ldb, long strideB, float* C, long ldc, long strideC);
-
 int sgemm_dispatch(int tA, int tB, long P, long M, long N, long K, const float* A, long lda, long strideA, const float* B,
                    long ldb, long strideB, float* C, long ldc, long strideC, int impl) {
   if (!require_runtime("sgemm")) return 1;
-  // one warp per output suits few outputs, or operands that both run along K in memory (its lanes read along K);
-  // the FMA tiles take the other products below the size at which the tensor-core kernels' fixed cost is repaid
-  const bool warp_per_output = impl == 5 || (impl == 0 && (M * N <= 2048 || (!tA && tB)));
-  if (warp_per_output) {
-    int rc = sgemm_small(tA, tB, P, M, N, K, A, lda, strideA, B, ldb, strideB, C, ldc, strideC);
-    if (rc >= 0) return rc;
-    if (impl == 5) return fail("sgemm: M=%ld N=%ld K=%ld is not a small product", M, N, K);
+  const Product<float> q = {tA, tB, P, M, N, K, A, lda, strideA, B, ldb, strideB, C, ldc, strideC};
+  if (impl == 5) {
+    const int rc = product_small(q);
+    return rc >= 0 ? rc : fail("sgemm: M=%ld N=%ld K=%ld is not a small product", M, N, K);
   }
-  if (impl == 0 || impl == 6) {
-    int rc = sgemm_tile16(tA, tB, P, M, N, K, A, lda, strideA, B, ldb, strideB, C, ldc, strideC);
-    if (rc >= 0) return rc;
-    if (impl == 6) return fail("sgemm: M=%ld N=%ld K=%ld is too large for the FMA-tile kernel", M, N, K);
-  }
+  if (impl == 6) return product_fma(q, true);
+  if (impl == 0 && product_is_fma(tA, tB, P, M, N, K)) return product_fma(q);
   if (impl != 1) {
     int rc = -1;
     if (impl != 3) rc = sgemm_tma(tA, tB, P, M, N, K, A, lda, strideA, B, ldb, strideB, C, ldc, strideC);
@@ -55,19 +45,23 @@ CGTB_API int cgtb_sgemm(int tA, int tB, long M, long N, long K, const float* A, 
                         long ldc, int impl) {
   return cgtb::sgemm_dispatch(tA, tB, 1, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, impl);
 }
-namespace cgtb {
-int sgemm_tile16_bias_add(int tA, int tB, long M, long N, long K, const float* A, long lda, const float* B, long ldb, const float* bias,
-                          const float* addend, long ldd, const float* addend_bias, float* C, long ldc);
-}
 CGTB_API int cgtb_sgemm_bias_add(int tA, int tB, long M, long N, long K, const float* A, long lda, const float* B, long ldb,
                                  const float* bias, const float* addend, long ldd, const float* addend_bias, float* C, long ldc) {
   if (!cgtb::require_runtime("cgtb_sgemm_bias_add")) return 1;
   if (addend_bias && !addend) return cgtb::fail("cgtb_sgemm_bias_add: addend_bias without addend");
-  const int rc = cgtb::sgemm_tile16_bias_add(tA, tB, M, N, K, A, lda, B, ldb, bias, addend, ldd, addend_bias, C, ldc);
-  if (rc < 0)
-    return cgtb::fail("cgtb_sgemm_bias_add: M=%ld N=%ld K=%ld (tA=%d tB=%d) is not a product of the FMA-tile kernel (M*N > 2048, M*N*K <= 2^25, "
+  // the kernels for few outputs have no such output stage
+  if (M * N <= 2048 || (!tA && tB) || K <= 0 || !cgtb::product_is_fma(tA, tB, 1, M, N, K))
+    return cgtb::fail("cgtb_sgemm_bias_add: M=%ld N=%ld K=%ld (tA=%d tB=%d) is not a product of the FMA-tile kernel (M*N > 2048, M*N*K <= 2^26, "
                       "not A.B^T); use cgtb_sgemm and add afterwards", M, N, K, tA, tB);
-  return rc;
+  cgtb::Product<float> q = {tA, tB, 1, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0};
+  q.sums = {bias, addend, ldd, addend_bias};
+  return cgtb::product_fma(q);
+}
+CGTB_API int cgtb_dgemm(int tA, int tB, long M, long N, long K, const double* A, long lda, const double* B, long ldb,
+                        double* C, long ldc) {
+  if (!cgtb::require_runtime("cgtb_dgemm")) return 1;
+  const cgtb::Product<double> q = {tA, tB, 1, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0};
+  return cgtb::product_fma(q);
 }
 CGTB_API int cgtb_sgemm_batched(int tA, int tB, long P, long M, long N, long K, const float* A, long lda, long strideA,
                                 const float* B, long ldb, long strideB, float* C, long ldc, long strideC, int impl) {
@@ -192,7 +186,7 @@ CGTB_API int cgtb_conv_bias_relu_ld(const float* col, long M, long K, long ldcol
   }
   // products that the dispatcher gives to the FMA kernels (below the tensor-core kernels' break-even size) take the
   // staged path below: the same product kernel, hence the same bits, as Mul22 followed by the separate output stage
-  if (M * (long)C * K > (1L << 25)) {
+  if (!cgtb::product_is_fma(0, 1, 1, M, C, K)) {
     // the tensor-core kernels apply the output stage to the accumulator tile when the product is not split
     // along K: no intermediate matrix at all
     cgtb::ConvEpilogue ep = {bias, y_nchw, mask_nchw, HW};

@@ -7,6 +7,7 @@
 // the CUDA kernels of this library. An array on the host is accepted only where the reference's
 // placement rule puts one: 0-d scalars and shape arithmetic (cgt/compilation.py:63-64); tensor
 // work on host arrays is refused rather than emulated.
+#include "products.h"
 #include "runtime.h"
 #include <cmath>
 #include <cstring>
@@ -225,8 +226,8 @@ struct FusedClosure { cgtbFusedProgram prog; long view_pitch[CGTB_FUSED_MAX_IN];
 OP_BYREF(cgtb_op_multi_fused_elwise) {
   const MultiFusedClosure* cl = (const MultiFusedClosure*)cl0;
   const int k = cl->k, n_in = cl->prog.n_in;
-  if (k < 1 || k > 24 || n_in < 1 || n_in > 4) { fail("MultiFusedElwise: unsupported group of %d tensors with %d inputs", k, n_in); return; }
-  const void* in[24 * 4];
+  if (k < 1 || k > 24 || n_in < 1 || n_in > 8) { fail("MultiFusedElwise: unsupported group of %d tensors with %d inputs", k, n_in); return; }
+  const void* in[24 * 8];
   void* out[24];
   long n[24];
   for (int t = 0; t < k; ++t) {
@@ -243,8 +244,11 @@ OP_BYREF(cgtb_op_multi_fused_elwise) {
   }
   cgtb_fused_elwise_multi(&cl->prog, k, n, in, out);
 }
-OP_BYREF(cgtb_op_fused_elwise) {
-  const cgtbFusedProgram* prog = (const cgtbFusedProgram*)cl0;
+// Pointers and broadcast extents of a FusedElwise's operands and results. `product`: index of an input that is not an
+// array (the element of a matrix product), or -1; `given` are the other inputs in order. false: an error was recorded.
+static bool chain_operands(const FusedClosure* cl0, cgtObject** given, cgtObject* write0, int product, long* n_out_elems, const void** in,
+                           long* bk, long* binner, void** out) {
+  const cgtbFusedProgram* prog = &cl0->prog;
   cgtArray* outs[CGTB_FUSED_MAX_OUT];
   if (prog->n_out == 1 && write0->kind() == cgtObject::ArrayKind) {
     outs[0] = ARR(write0);
@@ -253,40 +257,39 @@ OP_BYREF(cgtb_op_fused_elwise) {
     for (int q = 0; q < prog->n_out; ++q) outs[q] = ARR(tup->getitem(q));
   }
   cgtArray* w = outs[0];
-  const long n = w->size();
-  const void* in[CGTB_FUSED_MAX_IN];
-  void* out[CGTB_FUSED_MAX_OUT];
-  long bk[CGTB_FUSED_MAX_IN], binner[CGTB_FUSED_MAX_IN];
+  const long n = *n_out_elems = w->size();
   for (int q = 0; q < prog->n_out; ++q) {
-    if (outs[q]->size() != n || outs[q]->devtype() != cgtGPU) { fail("FusedElwise: outputs must be GPU arrays of one size"); return; }
+    if (outs[q]->size() != n || outs[q]->devtype() != cgtGPU) { fail("FusedElwise: outputs must be GPU arrays of one size"); return false; }
     out[q] = outs[q]->data();
   }
-  for (int k = 0; k < prog->n_in; ++k) {
-    cgtArray* x = ARR(reads[k]);
-    if (x->devtype() != cgtGPU) { fail("FusedElwise: operands must be on the GPU"); return; }
-    in[k] = x->data();
+  for (int k = 0, at = 0; k < prog->n_in; ++k) {
     bk[k] = binner[k] = 1;
+    in[k] = nullptr;
+    if (k == product) continue;
+    cgtArray* x = ARR(given[at++]);
+    if (x->devtype() != cgtGPU) { fail("FusedElwise: operands must be on the GPU"); return false; }
+    in[k] = x->data();
     const int kind = prog->in_kind[k];
     if ((kind == CGTB_FIN_F4 || kind == CGTB_FIN_I1) && x->size() != n) {
       fail("Shape error in a fused elementwise chain. You might be missing a call to cgt.broadcast(...)");
-      return;
+      return false;
     }
     if (kind == CGTB_FIN_VIEW_F4) {
-      const FusedClosure* fc = (const FusedClosure*)cl0;
+      const FusedClosure* fc = cl0;
       const long W = prog->view_width;
       if (W <= 0 || n % W != 0 || x->dtype() != cgt_f4 || x->size() != (n / W) * fc->view_pitch[k]) {
         fail("FusedElwise: operand %d is not the [%ld, %ld] matrix whose columns the chain reads", k, W > 0 ? n / W : 0, fc->view_pitch[k]);
-        return;
+        return false;
       }
       bk[k] = fc->view_pitch[k];
       binner[k] = fc->view_off[k];
     }
     if (kind == CGTB_FIN_BCAST_F4) {
-      if (x->ndim() != w->ndim()) { fail("FusedElwise: a broadcast operand must have the rank of the result"); return; }
+      if (x->ndim() != w->ndim()) { fail("FusedElwise: a broadcast operand must have the rank of the result"); return false; }
       int d0 = -1, d1 = -1;
       for (int d = 0; d < x->ndim(); ++d) {
         if (x->shape()[d] != 1) {
-          if (x->shape()[d] != w->shape()[d]) { fail("FusedElwise: broadcast operand does not match the result's shape"); return; }
+          if (x->shape()[d] != w->shape()[d]) { fail("FusedElwise: broadcast operand does not match the result's shape"); return false; }
           if (d0 < 0) d0 = d;
           d1 = d;
         }
@@ -294,7 +297,7 @@ OP_BYREF(cgtb_op_fused_elwise) {
       long kk = 1, inner = 1;
       if (d0 >= 0) {
         for (int d = d0; d <= d1; ++d) {
-          if (x->shape()[d] != w->shape()[d]) { fail("FusedElwise: the kept axes of a broadcast operand must be adjacent"); return; }
+          if (x->shape()[d] != w->shape()[d]) { fail("FusedElwise: the kept axes of a broadcast operand must be adjacent"); return false; }
           kk *= w->shape()[d];
         }
         for (int d = d1 + 1; d < w->ndim(); ++d) inner *= w->shape()[d];
@@ -303,7 +306,14 @@ OP_BYREF(cgtb_op_fused_elwise) {
       binner[k] = inner;
     }
   }
-  cgtb_fused_elwise(prog, n, in, bk, binner, out);
+  return true;
+}
+OP_BYREF(cgtb_op_fused_elwise) {
+  const FusedClosure* cl = (const FusedClosure*)cl0;
+  const void* in[CGTB_FUSED_MAX_IN];
+  void* out[CGTB_FUSED_MAX_OUT];
+  long bk[CGTB_FUSED_MAX_IN], binner[CGTB_FUSED_MAX_IN], n;
+  if (chain_operands(cl, reads, write0, -1, &n, in, bk, binner, out)) cgtb_fused_elwise(&cl->prog, n, in, bk, binner, out);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -324,6 +334,41 @@ OP_BYREF(cgtb_op_mul22) {
     cgtb_dgemm(cl->tA, cl->tB, M, N, K, (const double*)A->data(), lda, (const double*)B->data(), ldb, (double*)C->data(), ldc);
   else
     fail("Mul22: unsupported dtype %d", (int)A->dtype());
+}
+// Mul22Chain: (A, B, other inputs of the chain) -> the chain's results. The chain runs in the output stage of the FMA
+// product kernels; for a product that is not theirs it runs as a kernel of its own after the product.
+struct Mul22ChainClosure { FusedClosure chain; int product, tA, tB, variant; void* launcher; };
+OP_BYREF(cgtb_op_mul22_chain) {
+  const Mul22ChainClosure* cl = (const Mul22ChainClosure*)cl0;
+  const cgtbFusedProgram& fp = cl->chain.prog;
+  cgtArray *A = ARR(reads[0]), *B = ARR(reads[1]);
+  if (!all_gpu({A, B})) { fail("Mul22Chain: operands must be on the GPU"); return; }
+  const long lda = A->shape()[1], ldb = B->shape()[1];
+  const long M = A->shape()[cl->tA ? 1 : 0], K = A->shape()[cl->tA ? 0 : 1], Kb = B->shape()[cl->tB ? 1 : 0], N = B->shape()[cl->tB ? 0 : 1];
+  if (K != Kb || A->dtype() != B->dtype()) { fail("shape mismatch at matrix-matrix multiplication: (%ld x %ld) * (%ld x %ld)", M, K, Kb, N); return; }
+  const void* in[CGTB_FUSED_MAX_IN];
+  void* out[CGTB_FUSED_MAX_OUT];
+  long bk[CGTB_FUSED_MAX_IN], binner[CGTB_FUSED_MAX_IN], n;
+  if (!chain_operands(&cl->chain, reads + 2, write0, cl->product, &n, in, bk, binner, out)) return;
+  if (n != M * N) { fail("Mul22Chain: the chain's results have %ld elements, the product %ld", n, M * N); return; }
+  const Chain chain = {(ChainLauncher)cl->launcher, cl->variant, in, bk, binner, out};
+  auto go = [&](auto* tag) {
+    typedef typename std::remove_pointer<decltype(tag)>::type T;
+    Product<T> q = {cl->tA, cl->tB, 1, M, N, K, (const T*)A->data(), lda, 0, (const T*)B->data(), ldb, 0, nullptr, N, 0};
+    q.chain = &chain;
+    int rc = cl->launcher ? product_fma(q) : -1;
+    if (rc >= 0) return;
+    // no kernel was generated, or the extents are not those it was generated for
+    T* c = (T*)scratch_outer((size_t)n * sizeof(T));
+    if (!c) return;
+    if constexpr (sizeof(T) == 4) rc = sgemm_dispatch(cl->tA, cl->tB, 1, M, N, K, q.A, lda, 0, q.B, ldb, 0, c, N, 0, 0);
+    else rc = cgtb_dgemm(cl->tA, cl->tB, M, N, K, q.A, lda, q.B, ldb, c, N);
+    if (rc) return;
+    in[cl->product] = c;
+    cgtb_fused_elwise(&fp, n, in, bk, binner, out);
+  };
+  if (A->dtype() == cgt_f4) go((float*)nullptr);
+  else fail("Mul22Chain: unsupported dtype %d", (int)A->dtype());
 }
 // Mul22BiasAdd: (A, B, bias [1,N], addend [M,N], addend_bias [1,N]) -> (addend + addend_bias) + (A.B + bias)
 OP_BYREF(cgtb_op_mul22_bias_add) {

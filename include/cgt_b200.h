@@ -147,7 +147,7 @@ int cgtb_apply_byref(void* fptr, void* closure, int n, cgtbObject** reads, cgtbO
  * Replaces cblas_sgemm / cublasSgemm_v2 in cgt/core.py:2195-2222. 3xTF32 split on tcgen05 tensor
  * cores where the shape allows, fp32 FMA kernels otherwise and for products too small to repay the tensor-core
  * kernels' fixed cost. impl: 0 auto, 1 generic FMA kernel, 2 any tensor-core kernel, 3 register-fed tensor-core kernel,
- * 4 TMA-fed tensor-core kernel, 5 one warp per output (few outputs), 6 16 x 16 FMA tiles (M*N*K <= 2^25); a forced
+ * 4 TMA-fed tensor-core kernel, 5 one warp per output (few outputs), 6 FMA tiles; a forced
  * choice that does not accept the shape fails. */
 int cgtb_sgemm(int tA, int tB, long M, long N, long K, const float* A, long lda, const float* B, long ldb,
                float* C, long ldc, int impl);
@@ -160,9 +160,12 @@ int cgtb_sgemm_batched(int tA, int tB, long P, long M, long N, long K, const flo
  * do), in the product's output stage. bias, addend_bias: [N] rows; addend: [M, N] with row pitch ldd; each may be null
  * (addend_bias only with addend). The additions are plain float32 additions in exactly this association, so the result
  * has the bits of cgtb_sgemm followed by the three additions. Only products that cgtb_sgemm gives to its FMA-tile
- * kernel (M*N > 2048, M*N*K <= 2^25, not A.B^T); others are refused. */
+ * kernel (M*N > 2048, M*N*K <= 2^26, not A.B^T); others are refused. */
 int cgtb_sgemm_bias_add(int tA, int tB, long M, long N, long K, const float* A, long lda, const float* B, long ldb,
                         const float* bias, const float* addend, long ldd, const float* addend_bias, float* C, long ldc);
+/* Which of the FMA product kernels (cgt_product.h) this product runs in, -1 when it goes to the tensor cores; what an
+ * elementwise chain in its output stage is compiled for. */
+int cgtb_product_variant(int dtype, int tA, int tB, long M, long N, long K);
 int cgtb_dgemm(int tA, int tB, long M, long N, long K, const double* A, long lda, const double* B, long ldb,
                double* C, long ldc);
 
