@@ -78,7 +78,85 @@ def _function_listout(inputs, outputs, dbg=None, updates=None, givens=None):
     if dbg:
         raise core.Todo("debug functionality is broken")
     outputs = [_cgt().make_tuple(*x) if isinstance(x, tuple) else x for x in outputs]
-    return run_compilation_pipeline(inputs, outputs, updates, givens or [])
+    f = run_compilation_pipeline(inputs, outputs, updates, givens or [])
+    if core.get_config()["specialise_shapes"] and any(None in inp.get_fixed_shape() for inp in inputs if is_tensor(inp)):
+        return _SpecialisedByShape(f, inputs, outputs, updates, givens or [])
+    return f
+
+
+class _SpecialisedByShape(object):
+    """A function some of whose argument extents are open, and copies of it that were compiled for extents it is called
+    with again and again.
+
+    Almost every graph rewrite needs to know extents: with an open batch extent a training step of a small network is
+    30 launches and a dozen host instructions instead of 10 and none. So the third call with the same argument shapes
+    compiles the graph for them (tens of milliseconds) and later calls with these shapes go there; everything else, and
+    the first two calls with any shape, runs the general function. At most MOST copies are kept, the least recently used
+    one is dropped. All of them read and update the same shared variables."""
+    MOST, AFTER, WATCHED = 8, 3, 64
+
+    def __init__(self, general, inputs, outputs, updates, givens):
+        self._general = general
+        self._source = (inputs, outputs, updates, givens)
+        self._config = dict(core.get_config())
+        self._floatX = _cgt().floatX
+        self._calls, self._copies = {}, {}
+        self._frozen = False    # prefetch() in use: it must announce to the function that the next call runs
+
+    def _shapes(self, args):
+        try:
+            return tuple(a.shape for a in args)
+        except AttributeError:   # nested sequences, tuples
+            return None
+
+    def _pick(self, args, count):
+        key = self._shapes(args)
+        if key is None or len(args) != len(self._source[0]):
+            return self._general
+        f = self._copies.get(key)
+        if f is not None:
+            if len(self._copies) > 1:
+                self._copies[key] = self._copies.pop(key)
+            return f
+        if not count or self._frozen:
+            return self._general
+        n = self._calls.pop(key, 0) + 1
+        self._calls[key] = n
+        if len(self._calls) > self.WATCHED:
+            del self._calls[next(iter(self._calls))]
+        if n < self.AFTER:
+            return self._general
+        f = self._compile(key)
+        self._copies[key] = f
+        if len(self._copies) > self.MOST:
+            del self._copies[next(iter(self._copies))]
+        return f
+
+    def _compile(self, shapes):
+        (inputs, outputs, updates, givens) = self._source
+        if any(len(s) != inp.ndim for (s, inp) in zip(shapes, inputs)):
+            return self._general     # it reports the error
+        config = core.get_config()
+        saved, floatX = dict(config), _cgt().floatX
+        try:
+            config.update(self._config)   # the options that the function was compiled under
+            _cgt().set_precision("single" if self._floatX == "f4" else "double")
+            new = [core.Argument(inp.typ, name=inp.name, fixed_shape=tuple(int(d) for d in s), props=inp.props) for (s, inp) in zip(shapes, inputs)]
+            given = [(v, core.clone(w, dict(zip(inputs, new)))) for (v, w) in givens] + list(zip(inputs, new))
+            return run_compilation_pipeline(new, outputs, updates, given)
+        finally:
+            config.update(saved)
+            _cgt().set_precision("single" if floatX == "f4" else "double")
+
+    def __call__(self, *args):
+        return self._pick(args, True)(*args)
+
+    def prefetch(self, *args):
+        self._frozen = True
+        self._pick(args, False).prefetch(*args)
+
+    def __getattr__(self, name):
+        return getattr(self._general, name)
 
 
 # ================================================================
@@ -573,6 +651,82 @@ def fuse_slice_sums(outputs, updatetargs, node2shape):
     return _rewire(outputs, updatetargs, replace)
 
 
+def product_variant(dtype, tA, tB, M, N, K):
+    """Which of the FMA product kernels a product of these extents runs in (csrc/gemm_tile.cu), -1: none of them. Their
+    output stage can carry on with the result."""
+    from . import runtime
+    return int(runtime.lib().cgtb_product_variant(runtime.DTYPE_NUM[dtype], int(tA), int(tB), int(M), int(N), int(K)))
+
+
+def fuse_product_chains(outputs, updatetargs, updatesrcs, node2shape):
+    """An elementwise chain (FusedElwise, or a single elementwise node) one of whose inputs is a Mul22 that nothing else
+    reads -> Mul22Chain: the chain runs in the output stage of the product, element by element as before, so no bit
+    changes; one launch and one trip through memory less. For products of the FMA kernels. An update target may be such a
+    chain (p - lr * dW) unless the product itself reads the variable that is overwritten."""
+    all_out = list(outputs) + list(updatetargs)
+    nodes = core.topsorted(all_out)
+    children = defaultdict(list)
+    for node in nodes:
+        for par in node.parents:
+            children[par].append(node)
+    out_set = set(all_out)
+    overwrites = dict(zip(updatetargs, updatesrcs))
+    replace, taken = {}, set()
+    for node in nodes:
+        if node.is_input() or node.ndim not in (0, 2) and not is_tuple(node):
+            continue
+        if isinstance(node.op, core.FusedElwise):
+            chain = node.op
+        elif _fusable(node) and node.ndim == 2 and node.dtype == "f4":
+            kinds = [(2 if p.dtype == "f4" else 3) if p.ndim == 0 else (0 if p.dtype == "f4" else 1) for p in node.parents]
+            unary = isinstance(node.op, core.ElwiseUnary)
+            code = (core.UNARY_OPCODE if unary else core.BINARY_OPCODE)[node.op.opname]
+            distinct = list(dict.fromkeys(node.parents))
+            regs = [distinct.index(p) for p in node.parents]
+            if len(distinct) != len(node.parents):
+                kinds = [kinds[node.parents.index(p)] for p in distinct]
+            chain = core.FusedElwise([(1, code, regs[0], 0) if unary else (2, code, regs[0], regs[1])], kinds, [len(distinct)], ["f4"], 2,
+                                     kinds.index(0) if 0 in kinds else None, str(node.op),
+                                     static_shape=_static_shape(node2shape[node]))
+            if chain.static_shape is None:
+                continue
+        else:
+            continue
+        inputs = node.parents if chain is node.op else distinct
+        shp = node2shape[node][0] if is_tuple(node) else node2shape[node]
+        shp = _static_shape(shp)
+        if shp is None or len(shp) != 2:
+            continue
+        best = None
+        for (k, (src, kind)) in enumerate(zip(inputs, chain.in_kinds)):
+            if kind != 0 or src.is_input() or not isinstance(src.op, core.Mul22) or src in out_set or len(children[src]) != 1:
+                continue
+            if src.dtype != "f4" or any(p.dtype != "f4" for p in src.parents) or list(inputs).count(src) != 1:
+                continue
+            ashp = _static_shape(node2shape[src.parents[0]])
+            if ashp is None or _static_shape(node2shape[src]) != shp:
+                continue
+            K = ashp[0] if src.op.tA else ashp[1]
+            variant = product_variant("f4", src.op.tA, src.op.tB, shp[0], shp[1], K) if K >= 1 else -1
+            if variant < 0:
+                continue
+            if node in overwrites and overwrites[node] in src.parents:
+                continue
+            if best is None or K > best[1]:
+                best = (k, K, variant)
+        if best is None:
+            continue
+        product = inputs[best[0]]
+        others = [p for (k, p) in enumerate(inputs) if k != best[0]]
+        new = core.Result(core.Mul22Chain(product.op.tA, product.op.tB, chain, best[0], shp, best[2]), list(product.parents) + others)
+        node2shape[new] = node2shape[node]
+        new.props.update(node.props)
+        replace[node] = new
+    if not replace:
+        return list(outputs), list(updatetargs)
+    return _rewire(outputs, updatetargs, replace)
+
+
 def fuse_product_sums(outputs, updatetargs, node2shape):
     """z = (X + Repeat(b)) + (Mul22(h, U) + Repeat(c)), the pre-activation of a layer fed by two inputs (an unrolled
     recurrent cell forms it once per layer and time step) -> Mul22BiasAdd(h, U, c, X, b): the three additions run in
@@ -634,7 +788,7 @@ def fuse_product_sums(outputs, updatetargs, node2shape):
             if ashp is None or any(par.dtype != "f4" for par in m.parents):
                 continue
             K = ashp[0] if tA else ashp[1]
-            if M * N <= 2048 or (not tA and tB) or M * N * K > (1 << 25):
+            if M * N <= 2048 or (not tA and tB) or product_variant("f4", tA, tB, M, N, K) < 0:
                 continue     # not a product of the FMA-tile kernel
             new = core.Result(core.Mul22BiasAdd(tA, tB), [m.parents[0], m.parents[1], c_row, x, b_row])
             node2shape[new] = node2shape[z]
@@ -1121,6 +1275,8 @@ def fuse_elementwise(outputs, updatetargs, node2shape, rows=False):
             elif view is not None:
                 kind, src = 7, view[0]
                 views[len(inputs)] = (view[1], view[2])
+            elif _foldable_repeat(par) and (_static_shape(node2shape[par.parents[0]]) or (0,)).count(1) == par.ndim:
+                kind, src = 2, par.parents[0]   # one value: read like a scalar
             elif _foldable_repeat(par):
                 # the small operand is read directly; the Repeat node itself stays for whoever else uses it
                 kind, src = 4, par.parents[0]
@@ -1137,7 +1293,7 @@ def fuse_elementwise(outputs, updatetargs, node2shape, rows=False):
                 if par not in memset:
                     input_reg(par)
         n_in = len(inputs)
-        folded = sum(1 for k in in_kinds if k == 4)
+        folded = sum(1 for (k, src) in zip(in_kinds, inputs) if k == 4 or (k == 2 and src.ndim > 0))
         if len(mem) + folded < 2:
             return
         outs = [node for node in mem if node in out_set or any(c not in memset for c in children[node])]
@@ -1743,19 +1899,12 @@ def prebuild_fused_kernels(builders):
     """Generate and compile the fused-chain kernels of the given configurations into the library cache
     (no GPU needed: nvcc cross-compiles), so that a later run finds them instead of compiling."""
     from . import codegen
-    n = 0
+    ops = []
     for build in builders:
         cfg = build()
-        outs, _usrc, utargs, analysis = simplify_for_execution([cfg.loss] + list(cfg.extra_outputs), cfg.updates)
-        o2, u2 = apply_graph_rewrites(outs, utargs, analysis["node2shape"])
-        for node in core.topsorted(o2 + u2):
-            if node.is_input():
-                continue
-            if isinstance(node.op, core.FusedElwise) and codegen.fused_launcher(node.op):
-                n += 1
-            if isinstance(node.op, core.FusedRows) and codegen.rows_launcher(node.op):
-                n += 1
-    return n
+        eg = execution_graph(cfg.inputs, [cfg.loss] + list(cfg.extra_outputs), cfg.updates, [])[0]
+        ops += [ins.op for ins in eg.instrs if isinstance(ins, _Return)]
+    return codegen.generate_all(ops)
 
 
 # ================================================================
@@ -2093,7 +2242,7 @@ def merge_parameter_updates(eg, update_locs):
         if not isinstance(ins, ReturnByRef) or not isinstance(ins.op, core.FusedElwise) or ins.once:
             continue
         op = ins.op
-        if len(op.out_regs) != 1 or op.out_dtypes != ["f4"] or len(op.in_kinds) > 4 or any(k not in (0, 2, 3) for k in op.in_kinds):
+        if len(op.out_regs) != 1 or op.out_dtypes != ["f4"] or len(op.in_kinds) > 8 or any(k not in (0, 2, 3) for k in op.in_kinds):
             continue
         if ins.write_loc.index not in update_locs or ins.write_loc.devtype != "gpu":
             continue
@@ -2189,11 +2338,22 @@ def apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape):
     return outputs_simple, updatetargs_simple
 
 
-def run_compilation_pipeline(inputs, outputs, updates, givens):
+def rewrite_for_execution(outputs_simple, updatetargs_simple, updatesrcs, node2shape):
+    """apply_graph_rewrites, then the rewrites that need to know which variables the updates overwrite."""
+    config = core.get_config()
+    outputs_simple, updatetargs_simple = apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape)
+    # fuse_product_sums switches every use of the products' output stage
+    if config["fuse_elementwise"] and config["fuse_product_chains"] and config["fuse_product_sums"]:
+        outputs_simple, updatetargs_simple = fuse_product_chains(outputs_simple, updatetargs_simple, updatesrcs, node2shape)
+    return outputs_simple, updatetargs_simple
+
+
+def execution_graph(inputs, outputs, updates, givens):
+    """The instruction list, the simplified outputs and the memory locations of the nodes."""
     config = core.get_config()
     outputs_simple, updatesrcs, updatetargs_simple, analysis = simplify_for_execution(outputs, updates, givens)
     node2shape = analysis["node2shape"]
-    outputs_simple, updatetargs_simple = apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape)
+    outputs_simple, updatetargs_simple = rewrite_for_execution(outputs_simple, updatetargs_simple, updatesrcs, node2shape)
     all_out = outputs_simple + updatetargs_simple
 
     nodelist = core.topsorted(all_out)
@@ -2216,6 +2376,13 @@ def run_compilation_pipeline(inputs, outputs, updates, givens):
 
     if config["verbose"]:
         sys.stderr.write("begin\n" + "\n".join("%i.) \t%r" % (i, instr) for (i, instr) in enumerate(eg.instrs)) + "\nend\n")
+    return eg, outputs_simple, node2memloc
+
+
+def run_compilation_pipeline(inputs, outputs, updates, givens):
+    from . import codegen
+    (eg, outputs_simple, node2memloc) = execution_graph(inputs, outputs, updates, givens)
+    codegen.generate_all([ins.op for ins in eg.instrs if isinstance(ins, _Return)])
     return create_interpreter(inputs, outputs_simple, eg, node2memloc)
 
 

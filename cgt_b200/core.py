@@ -1186,6 +1186,9 @@ class FusedElwise(Op):
         return typs[0] if len(typs) == 1 else TupleType(*typs)
 
     def get_native_compile_info(self, input_types, devtype):
+        return NativeCompileInfo(None, prebuilt="cgtb_op_fused_elwise", closure_triples=self.closure(self._launcher()))
+
+    def closure(self, launcher):
         def arr(vals, n):
             vals = list(vals) + [0] * (n - len(vals))
             return (ctypes.c_int * n)(*vals)
@@ -1193,7 +1196,7 @@ class FusedElwise(Op):
             vals = list(vals) + [0] * (self.MAX_IN - len(vals))
             return (ctypes.c_long * self.MAX_IN)(*vals)
         code = {"f4": 11, "i1": 1}
-        return NativeCompileInfo(None, prebuilt="cgtb_op_fused_elwise", closure_triples=[
+        return [
             ("n_in", ctypes.c_int, len(self.in_kinds)),
             ("n_ops", ctypes.c_int, len(self.program)),
             ("n_out", ctypes.c_int, len(self.out_regs)),
@@ -1204,10 +1207,10 @@ class FusedElwise(Op):
             ("op_b", ctypes.c_int * self.MAX_OPS, arr([p[3] for p in self.program], self.MAX_OPS)),
             ("out_reg", ctypes.c_int * self.MAX_OUT, arr(self.out_regs, self.MAX_OUT)),
             ("out_dtype", ctypes.c_int * self.MAX_OUT, arr([code[d] for d in self.out_dtypes], self.MAX_OUT)),
-            ("launcher", ctypes.c_void_p, self._launcher()),
+            ("launcher", ctypes.c_void_p, launcher),
             ("view_width", ctypes.c_long, self.static_shape[1] if self.views else 0),
             ("view_pitch", ctypes.c_long * self.MAX_IN, larr([self.views.get(k, (0, 0))[1] for k in range(len(self.in_kinds))])),
-            ("view_off", ctypes.c_long * self.MAX_IN, larr([self.views.get(k, (0, 0))[0] for k in range(len(self.in_kinds))]))])
+            ("view_off", ctypes.c_long * self.MAX_IN, larr([self.views.get(k, (0, 0))[0] for k in range(len(self.in_kinds))]))]
 
     def _launcher(self):
         from . import codegen
@@ -1233,9 +1236,10 @@ class MultiFusedElwise(Op):
         self.k = int(k)
 
     def get_native_compile_info(self, input_types, devtype):
-        triples = list(self.fused.get_native_compile_info(input_types, devtype).closure_triples)
-        triples = [t for t in triples if t[0] not in ("launcher", "view_width", "view_pitch", "view_off")]
-        triples += [("launcher", ctypes.c_void_p, None), ("view_width", ctypes.c_long, 0), ("k", ctypes.c_int, self.k)]
+        from . import codegen
+        triples = self.fused.closure(codegen.multi_launcher(self))
+        triples = [t for t in triples if t[0] not in ("view_width", "view_pitch", "view_off")]
+        triples += [("view_width", ctypes.c_long, 0), ("k", ctypes.c_int, self.k)]
         return NativeCompileInfo(None, prebuilt="cgtb_op_multi_fused_elwise", closure_triples=triples)
 
     def __repr__(self):
@@ -1996,6 +2000,43 @@ class Mul22BiasAdd(Op):
         return "Mul22BiasAdd{%s,%s}" % ("T" if self.tA else "N", "T" if self.tB else "N")
 
 
+class Mul22Chain(Op):
+    """(A, B, other inputs of the chain) -> results of an elementwise chain on op(A).op(B) [M, N] and those inputs.
+
+    Not part of the reference's Op set: compilation.fuse_product_chains forms it from a FusedElwise one of whose inputs is
+    a product that nothing else reads (a layer's x.W + b with its nonlinearity, a gradient times the nonlinearity's
+    derivative, p - lr * dW). ``product``: the chain's input that is the product."""
+    available_impls = ("native_gpu",)
+
+    def __init__(self, tA, tB, chain, product, shape, variant):
+        assert chain.in_kinds[product] == 0
+        self.variant = int(variant)   # the product kernel that the chain is compiled into
+        self.tA, self.tB = bool(tA), bool(tB)
+        self.chain = chain
+        self.product = int(product)
+        self.shape = tuple(int(d) for d in shape)
+
+    def get_diff(self, num_inputs):
+        return [False] * num_inputs
+
+    def shp_apply(self, inputs):
+        shp = [cgt.constant(np.array(d, "i8")) for d in self.shape]
+        return shp if len(self.chain.out_regs) == 1 else tuple(list(shp) for _ in self.chain.out_regs)
+
+    def typ_apply(self, input_types):
+        return self.chain.typ_apply(None)
+
+    def get_native_compile_info(self, input_types, devtype):
+        from . import codegen
+        triples = self.chain.closure(None)
+        triples += [("product", ctypes.c_int, self.product), ("tA", ctypes.c_int, self.tA), ("tB", ctypes.c_int, self.tB),
+                    ("variant", ctypes.c_int, self.variant), ("launcher", ctypes.c_void_p, codegen.product_launcher(self))]
+        return NativeCompileInfo(None, prebuilt="cgtb_op_mul22_chain", closure_triples=triples)
+
+    def __repr__(self):
+        return "Mul22Chain{%s,%s %r}" % ("T" if self.tA else "N", "T" if self.tB else "N", self.chain)
+
+
 class BatchedMul22(Op):
     """Per-batch matrix product over the leading axis (cgt/core.py:2231-2288)."""
     available_impls = ("python", "native_cpu", "native_gpu")
@@ -2367,7 +2408,7 @@ _DEFAULTS = dict(
     debug=False, precision="single", backend="native", cache_dir="~/.cgt_b200_cache", enable_inplace_opt=True,
     enable_simplification=True, parallel=False, num_threads=1, force_python_impl=False, debug_cpp=False, verbose=False,
     # additions for this backend
-    devtype="gpu", device_index=0, use_cuda_graphs=True, fuse_elementwise=True, jit_fused_elementwise=True, fuse_conv_dgrad=True, fuse_conv_output=True, fuse_conv_grad_input=True, fuse_conv_implicit=True, fuse_conv_direct=True, fuse_flat_index_rows=True, hoist_filter_splits=True, split_gate_columns=True, fuse_product_sums=True, merge_parameter_updates=True, fuse_rows=True, fuse_slice_sums=True, fuse_slice_views=True, batch_summed_products=True,
+    devtype="gpu", device_index=0, use_cuda_graphs=True, fuse_elementwise=True, jit_fused_elementwise=True, fuse_conv_dgrad=True, fuse_conv_output=True, fuse_conv_grad_input=True, fuse_conv_implicit=True, fuse_conv_direct=True, fuse_flat_index_rows=True, hoist_filter_splits=True, split_gate_columns=True, fuse_product_sums=True, fuse_product_chains=True, specialise_shapes=True, merge_parameter_updates=True, fuse_rows=True, fuse_slice_sums=True, fuse_slice_views=True, batch_summed_products=True,
     pad_conv_columns=True, profile=False,
 )
 

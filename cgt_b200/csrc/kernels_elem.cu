@@ -282,7 +282,7 @@ CGTB_API int cgtb_fused_elwise(const cgtbFusedProgram* prog, long n, const void*
 // float32, inputs that are float32 tensors of the output's size or scalars. Same scalar templates as the single-tensor
 // kernel: same bits.
 constexpr int kMultiMaxTensors = 24;
-constexpr int kMultiMaxIn = 4;
+constexpr int kMultiMaxIn = 8;
 struct FusedMultiArgs {
   cgtbFusedProgram prog;
   int ntensors;
@@ -357,6 +357,15 @@ CGTB_API int cgtb_fused_elwise_multi(const cgtbFusedProgram* prog, int ntensors,
       return fail("cgtb_fused_elwise_multi: malformed program");
   }
   if (prog->out_reg[0] < 0 || prog->out_reg[0] >= prog->n_in + prog->n_ops) return fail("cgtb_fused_elwise_multi: bad output register");
+  if (prog->launcher) {
+    typedef int (*Launcher)(int, const long*, const void* const*, void* const*, void*);
+    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+    if (((Launcher)prog->launcher)(ntensors, n, in, out, (void*)rt().stream)) {
+      cudaGetLastError();
+      return fail("cgtb_fused_elwise_multi: the generated kernel failed to launch");
+    }
+    return 0;
+  }
   FusedMultiArgs a;
   a.prog = *prog;
   a.ntensors = ntensors;
