@@ -22,6 +22,7 @@ import pickle
 import string
 import subprocess
 import sys
+import threading
 from collections import defaultdict
 from io import StringIO
 
@@ -91,9 +92,12 @@ class _SpecialisedByShape(object):
     Almost every graph rewrite needs to know extents: with an open batch extent a training step of a small network is
     30 launches and a dozen host instructions instead of 10 and none. So the third call with the same argument shapes
     compiles the graph for them (tens of milliseconds) and later calls with these shapes go there; everything else, and
-    the first two calls with any shape, runs the general function. At most MOST copies are kept, the least recently used
-    one is dropped. All of them read and update the same shared variables."""
-    MOST, AFTER, WATCHED = 8, 3, 64
+    the first two calls with any shape, runs the general function. All copies read and update the same shared variables.
+
+    At most MOST copies are kept, the least recently used one is dropped; each drop doubles the number of calls that earn
+    a copy, so that a program which goes round many shapes soon runs the general function and compiles nothing. A copy
+    has buffers of its own: none is made while less than half of the device memory is free."""
+    MOST, AFTER, WATCHED = 4, 3, 64
 
     def __init__(self, general, inputs, outputs, updates, givens):
         self._general = general
@@ -101,6 +105,8 @@ class _SpecialisedByShape(object):
         self._config = dict(core.get_config())
         self._floatX = _cgt().floatX
         self._calls, self._copies = {}, {}
+        self._after = self.AFTER
+        self._lock = threading.Lock()
         self._frozen = False    # prefetch() in use: it must announce to the function that the next call runs
 
     def _shapes(self, args):
@@ -113,24 +119,33 @@ class _SpecialisedByShape(object):
         key = self._shapes(args)
         if key is None or len(args) != len(self._source[0]):
             return self._general
-        f = self._copies.get(key)
-        if f is not None:
-            if len(self._copies) > 1:
-                self._copies[key] = self._copies.pop(key)
+        with self._lock:
+            f = self._copies.get(key)
+            if f is not None:
+                if len(self._copies) > 1:
+                    self._copies[key] = self._copies.pop(key)
+                return f
+            if not count or self._frozen:
+                return self._general
+            n = self._calls.pop(key, 0) + 1
+            if n < self._after:
+                self._calls[key] = n
+                if len(self._calls) > self.WATCHED:
+                    del self._calls[next(iter(self._calls))]
+                return self._general
+            if not self._room():
+                return self._general
+            f = self._copies[key] = self._compile(key)
+            if len(self._copies) > self.MOST:
+                del self._copies[next(iter(self._copies))]
+                self._after *= 2
             return f
-        if not count or self._frozen:
-            return self._general
-        n = self._calls.pop(key, 0) + 1
-        self._calls[key] = n
-        if len(self._calls) > self.WATCHED:
-            del self._calls[next(iter(self._calls))]
-        if n < self.AFTER:
-            return self._general
-        f = self._compile(key)
-        self._copies[key] = f
-        if len(self._copies) > self.MOST:
-            del self._copies[next(iter(self._copies))]
-        return f
+
+    @staticmethod
+    def _room():
+        from . import runtime
+        free, total = runtime.device_memory()
+        return 2 * free >= total
 
     def _compile(self, shapes):
         (inputs, outputs, updates, givens) = self._source
@@ -144,6 +159,8 @@ class _SpecialisedByShape(object):
             new = [core.Argument(inp.typ, name=inp.name, fixed_shape=tuple(int(d) for d in s), props=inp.props) for (s, inp) in zip(shapes, inputs)]
             given = [(v, core.clone(w, dict(zip(inputs, new)))) for (v, w) in givens] + list(zip(inputs, new))
             return run_compilation_pipeline(new, outputs, updates, given)
+        except Exception:   # extents that do not fit together: the general function reports that as it always did
+            return self._general
         finally:
             config.update(saved)
             _cgt().set_precision("single" if floatX == "f4" else "double")

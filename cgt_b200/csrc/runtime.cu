@@ -276,6 +276,16 @@ CGTB_API int cgtb_pool_trim(void) {
 }
 CGTB_API long cgtb_kernel_launches(void) { return g_kernel_launches.load(); }
 CGTB_API int cgtb_sm_count(void) { return g_rt.sm_count; }
+CGTB_API int cgtb_device_memory(long* free_bytes, long* total_bytes) {
+  if (!require_runtime("cgtb_device_memory")) return 1;
+  size_t f = 0, t = 0;
+  CGTB_CUDA_TRY(cudaMemGetInfo(&f, &t));
+  long reserved = 0, in_use = 0, high = 0, mallocs = 0;
+  if (cgtb_pool_stats(&reserved, &in_use, &high, &mallocs)) return 1;
+  *free_bytes = (long)f + reserved - in_use;
+  *total_bytes = (long)t;
+  return 0;
+}
 
 // ================================================================== C ABI: memory
 CGTB_API void* cgtb_alloc(int devtype, long nbytes) {

@@ -39,7 +39,7 @@ def _declare(lib):
         "cgtb_init": (ci, [ci]), "cgtb_initialized": (ci, []), "cgtb_device": (ci, []),
         "cgtb_last_error": (ctypes.c_char_p, []), "cgtb_clear_error": (None, []), "cgtb_synchronize": (ci, []),
         "cgtb_stream": (vp, []), "cgtb_pool_stats": (ci, [c_long_p] * 4), "cgtb_pool_trim": (ci, []),
-        "cgtb_kernel_launches": (cl, []), "cgtb_sm_count": (ci, []),
+        "cgtb_kernel_launches": (cl, []), "cgtb_sm_count": (ci, []), "cgtb_device_memory": (ci, [c_long_p] * 2),
         "cgtb_event_new": (vp, []), "cgtb_event_record": (ci, [vp]),
         "cgtb_event_elapsed_ms": (ci, [vp, vp, ctypes.POINTER(ctypes.c_float)]), "cgtb_event_free": (None, [vp]),
         "cgtb_l2_flush": (ci, []), "cgtb_selftest_refused_launch": (ci, []),
@@ -364,6 +364,14 @@ def device_array(nparr):
     w = ArrayWrapper.from_numpy(nparr, "gpu")
     w.materialize()
     return w
+
+
+def device_memory():
+    """(free, total) bytes of the GPU; what the runtime's pool holds and nothing uses counts as free."""
+    ensure_init()
+    free, total = ctypes.c_long(0), ctypes.c_long(0)
+    check(lib().cgtb_device_memory(ctypes.byref(free), ctypes.byref(total)), "device memory")
+    return free.value, total.value
 
 
 def pinned_empty(shape, dtype):

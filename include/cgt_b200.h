@@ -35,6 +35,7 @@ int cgtb_pool_stats(long* reserved_bytes, long* in_use_bytes, long* high_water_b
 int cgtb_pool_trim(void);                  /* return cached blocks to the driver */
 long cgtb_kernel_launches(void);           /* kernels launched by this library since load */
 int cgtb_sm_count(void);
+int cgtb_device_memory(long* free_bytes, long* total_bytes); /* the pool's idle blocks count as free */
 
 /* Timing on the runtime stream (CUDA events) and an L2 flush for benchmarks. */
 void* cgtb_event_new(void);

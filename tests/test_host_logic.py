@@ -553,3 +553,26 @@ def test_checkpoint_file_round_trip(tmp_path):
     pc.set_value_flat(theta * 2)
     for (p, b) in zip(other.params, before):
         assert np.array_equal(p.op.get_value(), b * 2)
+
+
+# ------------------------------------------------------------------------------------------------
+# copies compiled per argument shape; the steps of unrolled networks
+# ------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("n_shapes", [1, 3, 12])
+def test_copies_per_shape_do_not_thrash(monkeypatch, n_shapes):
+    """A program that goes round more shapes than copies are kept compiles a bounded number of times."""
+    compiled = []
+    monkeypatch.setattr(compilation, "run_compilation_pipeline", lambda inputs, *a: compiled.append(inputs) or (lambda *args: "copy"))
+    monkeypatch.setattr(compilation._SpecialisedByShape, "_room", staticmethod(lambda: True))
+    x = cgt.matrix("x")
+    f = compilation._SpecialisedByShape(lambda *args: "general", [x], [x * 2.0], None, [])
+    args = [np.zeros((4 + i, 3), "f4") for i in range(n_shapes)]
+    for _ in range(100):
+        got = [f(a) for a in args]
+    assert len(f._copies) <= f.MOST
+    if n_shapes <= f.MOST:
+        assert set(got) == {"copy"} and len(compiled) == n_shapes
+    else:   # the n-th copy that drops another costs 3 * 2^n calls with its shape
+        assert len(compiled) <= f.MOST + n_shapes * 6
+    monkeypatch.setattr(compilation._SpecialisedByShape, "_room", staticmethod(lambda: False))
+    assert f(np.zeros((99, 3), "f4")) == "general" and f([[1.0, 2.0]]) == "general"
