@@ -322,6 +322,170 @@ def product_launcher(op):
     return _generated_launcher(product_source(op), "product_", "cgtb_product_launch", "a chain in a product's output stage")
 
 
+def recurrence_plan(R, H, KA, N, n_act):
+    """How a Recurrence is dealt out, or None when it does not fit. A cluster of C blocks owns RB rows through all steps;
+    block c of it computes the N / H columns of UH of the H units. Its slice of W stays in registers for the whole launch:
+    256 threads, one column each, KG of them sharing a column's K, KT values per thread. Chosen for the fewest
+    multiply-adds per thread and step, RB * KT; of equals the smallest cluster, whose barrier is the cheapest."""
+    NG, best = N // H, None
+    for C in (1, 2, 4, 8):
+        UH = -(-H // C)
+        NC = NG * UH
+        if NC > 256 or (C > 1 and UH * (C - 1) >= H):
+            continue
+        KG = 256 // NC
+        KT = -(-(-(-KA // KG)) // 4) * 4
+        KG = -(-KA // KT)
+        RB = -(-R // (128 // C))
+        shared = 4 * (2 * RB * KG * KT + KG * RB * NC)
+        # 72 weights per thread leave registers for the sums and the chain; 8 rows: beyond that, a launch per step over
+        # the whole batch has enough work per block
+        if KT > 72 or RB > 8 or RB * UH > 256 or shared > 46 * 1024:
+            continue
+        if best is None or RB * KT < best[0]:
+            best = (RB * KT, dict(C=C, UH=UH, NC=NC, KG=KG, KT=KT, RB=RB, NG=NG))
+    return best and best[1]
+
+
+def recurrence_source(op):
+    """CUDA source of the kernel for one Recurrence (plan: recurrence_plan). One step: every thread multiplies its KT
+    weights (registers) with the rows' act (shared memory, broadcast reads), the K groups' partial sums meet in shared
+    memory, one thread per (row, unit) adds them in order, runs the chain and writes its part of the next act into the
+    shared memory of all blocks of the cluster; a cluster barrier ends the step. The act is double-buffered, so one barrier
+    per step is enough; the chain's other operands are loaded a step ahead.
+
+    Bound by that serial chain, not by operations: the FMAs of a step (2 rows x 128 columns x 128 per block) take about
+    300 cycles."""
+    p = recurrence_plan(op.R, op.H, op.KA, op.N, len(op.act_spec))
+    chain, n_in = op.chain, len(op.chain.in_kinds)
+    states = sorted(op.state)
+    per = int(op.bias) + len(op.external) + len(op.kept) + int(op.keep_act)
+    ext0 = int(op.bias)
+    regs, loads = [], []   # (type, name) of the operands that are loaded a step ahead
+    if op.bias:
+        for g in range(p["NG"]):
+            regs.append("x%d" % g)
+            loads.append("((const float*)q[0])[row * %d + %d + j]" % (op.N, g * op.H))
+    for (pos, k) in enumerate(op.external):
+        kind, src = chain.in_kinds[k], "q[%d]" % (ext0 + pos)
+        regs.append("e%d" % k)
+        loads.append({0: "((const float*)%s)[row * %d + j]" % (src, op.H), 2: "((const float*)%s)[0]" % src,
+                      3: "(float)((const long*)%s)[0]" % src,
+                      7: "((const float*)%s)[row * %d + %d + j]" % ((src,) + chain.views.get(k, (0, 0))[::-1])}[kind])
+    L = ['namespace {',
+         'constexpr int R = %d, H = %d, KA = %d, N = %d, C = %d, UH = %d, NC = %d, KG = %d, KT = %d, RB = %d, PER = %d;'
+         % (op.R, op.H, op.KA, op.N, p["C"], p["UH"], p["NC"], p["KG"], p["KT"], p["RB"], per),
+         'constexpr int KP = KG * KT, kPointers = %d;' % min(op.MAX_POINTERS, max(256, 1 << (per * op.steps - 1).bit_length())),
+         'struct Job { const void* fixed[20]; int steps; const void* p[kPointers]; };',
+         '// Warps come here from divergent code: they gather first, and every thread arrives for itself (no .aligned). Reached',
+         '// without any condition in every step, the last one included: under one (s + 1 < steps, which the chain tests as well)',
+         '// the two halves of a warp may take different ways to it.',
+         '__device__ __forceinline__ void step_barrier() {',
+         '  __syncwarp();',
+         '  if (C > 1) asm volatile("barrier.cluster.arrive.release;\\n\\tbarrier.cluster.wait.acquire;" ::: "memory");',
+         '  else __syncthreads();', '}',
+         '__device__ __forceinline__ void store_peer(float* own, int block, float v) {',
+         '  if (C == 1) { *own = v; return; }',
+         '  unsigned at;',
+         '  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((unsigned)__cvta_generic_to_shared(own)), "r"(block));',
+         '  asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(at), "f"(v) : "memory");', '}',
+         '__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(256) recurrence_kernel(const __grid_constant__ Job a) {',
+         '  __shared__ __align__(16) float act[2][RB][KP];',
+         '  __shared__ float part[KG][RB][NC];',
+         '  const int tid = threadIdx.x, u0 = (int)(blockIdx.x % C) * UH, row0 = (int)(blockIdx.x / C) * RB;',
+         '  const int col = tid % NC, kg = tid / NC;',
+         '  const bool multiplies = kg < KG;',
+         '  const float* W = (const float*)a.fixed[1];',
+         '  float w[KT];',
+         '  {',
+         '    const int unit = u0 + col % UH, n = (col / UH) * H + unit;',
+         '#pragma unroll',
+         '    for (int k = 0; k < KT; ++k) {',
+         '      const int kk = kg * KT + k;',
+         '      w[k] = multiplies && unit < H && kk < KA ? W[%s] : 0.0f;' % ("n * KA + kk" if op.tB else "kk * N + n"),
+         '    }', '  }',
+         '  for (int i = tid; i < RB * KP; i += 256) {',
+         '    const int r = i / KP, k = i % KP;',
+         '    act[0][r][k] = row0 + r < R && k < KA ? ((const float*)a.fixed[0])[(row0 + r) * KA + k] : 0.0f;',
+         '    act[1][r][k] = 0.0f;',
+         '  }',
+         '  const int rr = tid / UH, u = tid % UH, j = u0 + u, row = row0 + rr;',
+         '  const bool live = rr < RB && j < H && row < R;']
+    if op.bias:
+        for g in range(p["NG"]):
+            L.append('  const float b%d = live ? ((const float*)a.fixed[2])[%d + j] : 0.0f, c%d = live ? ((const float*)a.fixed[3])[%d + j] : 0.0f;'
+                     % (g, g * op.H, g, g * op.H))
+    for (pos, k) in enumerate(states):
+        L.append('  float t%d = live ? ((const float*)a.fixed[%d])[row * H + j] : 0.0f;' % (k, 2 + 2 * op.bias + pos))
+    L += ['  float %s;' % ", ".join("%s = 0.0f, next_%s = 0.0f" % (r, r) for r in regs)] if regs else []
+    fetch = ['      next_%s = %s;' % (r, ld) for (r, ld) in zip(regs, loads)]
+    L += ['  if (live) {', '    const void* const* q = a.p;', '    (void)q;'] + fetch + ['  }',
+          '  step_barrier();',
+          '  for (int s = 0; s < a.steps; ++s) {',
+          '    const void* const* now = a.p + s * PER;', '    (void)now;']
+    L += ['    %s = next_%s;' % (r, r) for r in regs]
+    L += ['    if (live) {  // a step ahead; the last one again at the end', '      const void* const* q = a.p + (s + 1 < a.steps ? s + 1 : s) * PER;',
+          '      (void)q;'] + fetch + ['    }',
+          '    if (multiplies) {',
+          '      float sum[RB];',
+          '#pragma unroll',
+          '      for (int r = 0; r < RB; ++r) sum[r] = 0.0f;',
+          '      const float* x = &act[s & 1][0][kg * KT];',
+          '#pragma unroll',
+          '      for (int k = 0; k < KT; k += 4) {',
+          '#pragma unroll',
+          '        for (int r = 0; r < RB; ++r) {',
+          '          const float4 v = *reinterpret_cast<const float4*>(x + r * KP + k);',
+          '          sum[r] = fmaf(v.x, w[k], sum[r]);', '          sum[r] = fmaf(v.y, w[k + 1], sum[r]);',
+          '          sum[r] = fmaf(v.z, w[k + 2], sum[r]);', '          sum[r] = fmaf(v.w, w[k + 3], sum[r]);',
+          '        }', '      }',
+          '#pragma unroll',
+          '      for (int r = 0; r < RB; ++r) part[kg][r][col] = sum[r];',
+          '    }',
+          '    __syncthreads();',
+          '    if (live) {']
+    for g in range(p["NG"]):
+        L += ['      float z%d = part[0][rr][%d + u];' % (g, g * p["UH"]), '#pragma unroll',
+              '      for (int k = 1; k < KG; ++k) z%d += part[k][rr][%d + u];' % (g, g * p["UH"])]
+        if op.bias:
+            L.append('      z%d = (x%d + c%d) + (z%d + b%d);' % (g, g, g, g, g))
+    for k in range(n_in):
+        src = "z%d" % (op.z_inputs[k] // op.H) if k in op.z_inputs else "t%d" % k if k in op.state else "e%d" % k
+        L.append('      const float r%d = %s;' % (k, src))
+    for (i, (arity, code, x, y)) in enumerate(chain.program):
+        L.append('      const float r%d = %s;' % (n_in + i, "unary_apply<float, float>(%d, r%d)" % (code, x) if arity == 1 else
+                                                  "binary_apply<float, float, float>(%d, r%d, r%d)" % (code, x, y)))
+    at = ext0 + len(op.external)
+    for (pos, q) in enumerate(op.kept):
+        L.append('      ((float*)now[%d])[row * H + j] = r%d;' % (at + pos, chain.out_regs[q]))
+    if op.keep_act:
+        for (q, off) in op.act_spec:
+            L.append('      ((float*)now[%d])[row * KA + %d + j] = r%d;' % (at + len(op.kept), off, chain.out_regs[q]))
+    for k in states:
+        L.append('      t%d = r%d;' % (k, chain.out_regs[op.state[k]]))
+    L += ['      float* dst = &act[(s + 1) & 1][rr][j];',
+          '#pragma unroll', '      for (int c = 0; c < C; ++c) {']
+    L += ['        store_peer(dst + %d, c, r%d);' % (off, chain.out_regs[q]) for (q, off) in op.act_spec]
+    L += ['      }', '    }',
+          '    step_barrier();',
+          '  }', '}', '}  // namespace',
+          'extern "C" __attribute__((visibility("default"))) int cgtb_recurrence_launch(int steps, const void* const* fixed,',
+          '    const void* const* per_step, void* stream) {',
+          '  if (steps < 1 || steps * PER > kPointers) return 1;',
+          '  Job a;',
+          '  for (int k = 0; k < %d; ++k) a.fixed[k] = fixed[k];' % (2 + 2 * op.bias + len(states)),
+          '  a.steps = steps;',
+          '  for (int k = 0; k < steps * PER; ++k) a.p[k] = per_step[k];',
+          '  recurrence_kernel<<<C * ((R + RB - 1) / RB), 256, 0, (cudaStream_t)stream>>>(a);',
+          '  return cudaPeekAtLastError() != cudaSuccess;', '}']
+    return _FUSED_HEAD + "\n".join(L) + "\n"
+
+
+def recurrence_launcher(op):
+    """Address of the generated launcher for a Recurrence, or None: its steps stay separate launches then."""
+    return _generated_launcher(recurrence_source(op), "recurrence_", "cgtb_recurrence_launch", "the steps of a recurrent network")
+
+
 _fused_libs = {}
 
 
@@ -342,8 +506,10 @@ def generate_all(ops):
     """Generate and compile the kernels of these Ops that are not in the cache yet, several compilers at a time; the
     number of Ops that have a generated kernel."""
     import concurrent.futures
-    makers = {core.FusedElwise: fused_launcher, core.MultiFusedElwise: multi_launcher, core.FusedRows: rows_launcher, core.Mul22Chain: product_launcher}
-    sources = {core.FusedElwise: fused_source, core.MultiFusedElwise: multi_source, core.FusedRows: rows_source, core.Mul22Chain: product_source}
+    makers = {core.FusedElwise: fused_launcher, core.MultiFusedElwise: multi_launcher, core.FusedRows: rows_launcher, core.Mul22Chain: product_launcher,
+              core.Recurrence: recurrence_launcher}
+    sources = {core.FusedElwise: fused_source, core.MultiFusedElwise: multi_source, core.FusedRows: rows_source, core.Mul22Chain: product_source,
+               core.Recurrence: recurrence_source}
     todo, n = {}, 0
     for op in ops:
         if type(op) in makers:

@@ -744,6 +744,320 @@ def fuse_product_chains(outputs, updatetargs, updatesrcs, node2shape):
     return _rewire(outputs, updatetargs, replace)
 
 
+def batch_row_chains(outputs, updatetargs, node2shape):
+    """FusedRows nodes of one program whose matrices are the consecutive leading slices of whole arrays, whose other
+    operands are the same and none of which needs another's result (the softmax and its pullback at every time step of
+    an unrolled network) -> ONE FusedRows over the whole arrays, every original result a LeadingSlice view of its result.
+    Rows are independent of each other, so no bit changes. Fifty launches on [64, 65] take 150 us, the one 4 us."""
+    all_out = list(outputs) + list(updatetargs)
+    nodes = core.topsorted(all_out)
+    children = defaultdict(list)
+    for node in nodes:
+        for par in node.parents:
+            children[par].append(node)
+    out_set = set(all_out)
+
+    def slice_of(node):
+        """(array, first row, rows of the array) when `node` is a leading slice of it, through reshapes that keep its rows"""
+        shp = _static_shape(node2shape[node])
+        while not node.is_input() and isinstance(node.op, core.Reshape):
+            node = node.parents[0]
+        if shp is None or node.is_input() or not isinstance(node.op, core.LeadingSlice):
+            return None
+        (x, start, stop) = node.parents
+        if not isinstance(start.op, core.Constant) or not isinstance(stop.op, core.Constant):
+            return None
+        xshp = _static_shape(node2shape[x])
+        if xshp is None or len(shp) == 0:
+            return None
+        per = int(np.prod(xshp[1:], dtype=np.int64))      # elements per leading index, the slice begins at one
+        row = int(np.prod(shp[1:], dtype=np.int64))
+        if row < 1 or (int(start.op.value) * per) % row or (xshp[0] * per) % row:
+            return None
+        if int(stop.op.value) * per - int(start.op.value) * per != shp[0] * row:
+            return None
+        return x, int(start.op.value) * per // row, xshp[0] * per // row, shp
+
+    def plain(node):
+        """(kind, operand of node) of a FusedRows, a constant array of one value (folded at compile time) as a scalar"""
+        out = []
+        for (par, kind) in zip(node.parents, node.op.in_kinds):
+            if kind in (0, 5, 6) and not par.is_input() and isinstance(par.op, core.Constant) and par.dtype == "f4":
+                v = np.asarray(par.op.value)
+                if v.size and v.tobytes() == v.reshape(-1)[:1].tobytes() * v.size:
+                    (kind, par) = (2, core.cgt.constant(v.reshape(-1)[0]))
+                    node2shape[par] = []
+            out.append((kind, par))
+        return out
+
+    def same(node):
+        """what two operands have in common that hold the same value"""
+        if not node.is_input() and isinstance(node.op, core.Constant) and np.size(node.op.value) == 1:
+            v = np.asarray(node.op.value)
+            return (v.dtype.str, v.shape, v.tobytes())
+        return id(node)
+
+    groups = defaultdict(list)
+    for node in nodes:
+        if node.is_input() or not isinstance(node.op, core.FusedRows) or node in out_set:
+            continue
+        key, starts = [tuple(node.op.program), tuple(node.op.in_kinds), tuple(node.op.out_regs), tuple(node.op.out_cols), node.op.C], set()
+        for (kind, par) in plain(node):
+            if kind in (0, 5, 8):
+                sl = slice_of(par)
+                if sl is None or par in out_set:
+                    break
+                starts.add(sl[1])
+                key.append((id(sl[0]), sl[2], sl[3]))
+            else:
+                key.append(same(par))
+        else:
+            if len(starts) == 1:
+                groups[tuple(key)].append((starts.pop(), node))
+    replace = {}
+    for members in groups.values():
+        members.sort(key=lambda m: m[0])
+        first = members[0][1]
+        operands = plain(first)
+        by_row = [par for (kind, par) in operands if kind in (0, 5, 8)]
+        R, whole = _static_shape(node2shape[by_row[0]])[0], slice_of(by_row[0])
+        if len(members) < 2 or [m[0] for m in members] != [R * t for t in range(len(members))] or whole[2] != R * len(members):
+            continue
+        if any(_static_shape(node2shape[par])[0] != R for par in by_row):
+            continue
+        reached = {m[1] for m in members}
+        for node in nodes:
+            if any(p in reached for p in node.parents):
+                if any(node is m[1] for m in members):
+                    break
+                reached.add(node)
+        else:
+            rows = core.cgt.constant(np.array(whole[2], "i8"))
+            inputs = []
+            for (kind, par) in operands:
+                if kind in (0, 5, 8):
+                    (x, _first, _rows, shp) = slice_of(par)
+                    shape = [rows] + [core.cgt.constant(np.array(d, "i8")) for d in shp[1:]]
+                    par = core.Result(core.Reshape(), [x] + shape)
+                    node2shape[par] = shape
+                inputs.append(par)
+            op = first.op
+            new = core.Result(core.FusedRows(op.program, [kind for (kind, _par) in operands], op.out_regs, op.out_cols, op.C,
+                                             [kind in (0, 5, 8) for (kind, _par) in operands].index(True), op.descr), inputs)
+            shapes = tuple([rows, core.cgt.constant(np.array(1 if col else op.C, "i8"))] for col in op.out_cols)
+            node2shape[new] = shapes if is_tuple(first) else shapes[0]
+            for (t, (_start, m)) in enumerate(members):
+                for old in (children[m] if is_tuple(m) else [m]):
+                    src = new
+                    if is_tuple(m):
+                        src = core.Result(core.TupleIndex(old.op.idx), [new])
+                        node2shape[src] = shapes[old.op.idx]
+                    view = core.Result(core.LeadingSlice(), [src, core.cgt.constant(np.array(t * R, "i8")), core.cgt.constant(np.array((t + 1) * R, "i8"))])
+                    node2shape[view] = node2shape[old]
+                    view.props.update(old.props)
+                    replace[old] = view
+    if not replace:
+        return list(outputs), list(updatetargs)
+    return _rewire(outputs, updatetargs, replace)
+
+
+def fuse_recurrences(outputs, updatetargs, node2shape):
+    """Consecutive steps of an unrolled recurrent network, forward or differentiated -> Recurrence, one launch.
+
+    A step is a FusedElwise over [R, H] that reads, besides other things, a product (Mul22, Mul22BiasAdd) of the state
+    with one matrix; the state of the next step is one of its results, or a ScatterCols that places several of them. Steps
+    belong together while chain, matrix and the way in which one feeds the next are the same; the first and the last step
+    of a network usually differ and stay as they are. A step whose other operands depend on an earlier step of the same
+    group by another way starts a new group. Products and chains that run as they are take two to three launches of 3 us
+    per step, half of it latency; a step of the one launch takes about 0.7 us."""
+    from . import codegen
+    refused = set()
+    while True:
+        all_out = list(outputs) + list(updatetargs)
+        nodes = core.topsorted(all_out)
+        children = defaultdict(list)
+        for node in nodes:
+            for par in node.parents:
+                children[par].append(node)
+        group = _find_recurrence(nodes, children, set(all_out), set(updatetargs), node2shape, refused)
+        if group is None:
+            return list(outputs), list(updatetargs)
+        (steps, op, inputs, results) = group
+        if codegen.recurrence_launcher(op) is None:
+            refused.update(s["chain"] for s in steps)
+            continue
+        new = core.Result(op, inputs)
+        first = node2shape[steps[0]["chain"]]
+        element = first[0] if is_tuple(steps[0]["chain"]) else first
+        act = node2shape[steps[0]["product"].parents[0]]
+        node2shape[new] = tuple(list(shp) for shp in ([element] * len(op.kept) + [act] * op.keep_act) * op.steps)
+        replace = {}
+        for (i, old) in results:
+            part = core.Result(core.TupleIndex(i), [new])
+            node2shape[part] = node2shape[old]
+            part.props.update(old.props)
+            replace[old] = part
+        outputs, updatetargs = _rewire(outputs, updatetargs, replace)
+
+
+def _recurrence_step(node, children, out_set, node2shape):
+    """What `node` is as a step of a recurrent network, or None."""
+    if node.is_input() or not isinstance(node.op, core.FusedElwise) or node in out_set:
+        return None
+    op = node.op
+    shp = node2shape[node][0] if is_tuple(node) else node2shape[node]
+    shp = _static_shape(shp)
+    if shp is None or len(shp) != 2 or any(d != "f4" for d in op.out_dtypes) or any(k not in (0, 2, 3, 7) for k in op.in_kinds):
+        return None
+    (R, H) = shp
+    found = []
+    for p in dict.fromkeys(node.parents):
+        if p.is_input() or not isinstance(p.op, (core.Mul22, core.Mul22BiasAdd)) or p.op.tA or p in out_set or p.dtype != "f4":
+            continue
+        if any(q.dtype != "f4" for q in p.parents) or set(children[p]) != {node}:
+            continue
+        pshp, ashp = _static_shape(node2shape[p]), _static_shape(node2shape[p.parents[0]])
+        if pshp is None or ashp is None or pshp[0] != R or pshp[1] % H != 0 or min(R, H, ashp[1]) < 1:
+            continue
+        cols = {}
+        for (k, q) in enumerate(node.parents):
+            if q is p:
+                cols[k] = op.views[k][0] if op.in_kinds[k] == 7 else 0
+        if any(c % H != 0 or c >= pshp[1] for c in cols.values()) or any(op.in_kinds[k] == 0 and pshp[1] != H for k in cols):
+            continue
+        found.append((p, cols, pshp[1], ashp[1]))
+    if len(found) != 1:
+        return None
+    (p, cols, N, KA) = found[0]
+    bias = isinstance(p.op, core.Mul22BiasAdd)
+    fixed = (p.parents[1],) + ((p.parents[2], p.parents[4]) if bias else ())
+    sig = (tuple(op.program), tuple(op.in_kinds), tuple(op.out_regs), tuple(sorted(op.views.items())), (R, H, N, KA), p.op.tB, bias,
+           fixed, tuple(sorted(cols.items())))
+    return dict(chain=node, product=p, cols=cols, R=R, H=H, N=N, KA=KA, bias=bias, fixed=fixed, sig=sig)
+
+
+def _find_recurrence(nodes, children, out_set, update_set, node2shape, refused):
+    """(steps, Recurrence Op, its inputs, [(result index, node it stands for)]) of one group of steps, or None."""
+    from . import codegen
+    steps = {}
+    for node in nodes:
+        if node not in refused and not node.is_input() and isinstance(node.op, core.FusedElwise):
+            st = _recurrence_step(node, children, out_set, node2shape)
+            if st is not None:
+                steps[node] = st
+
+    def result_of(node):
+        """(chain node, result number) that `node` is"""
+        if node in steps and not is_tuple(node):
+            return node, 0
+        if not node.is_input() and isinstance(node.op, core.TupleIndex) and node.parents[0] in steps:
+            return node.parents[0], node.op.idx
+        return None, None
+
+    def act_of(act, st):
+        """(chain node, [(result, first column)]) whose results `act` is made of"""
+        if result_of(act)[0] is not None:
+            (prev, q) = result_of(act)
+            return (prev, [(q, 0)]) if st["KA"] == st["H"] else (None, None)
+        if act.is_input() or not isinstance(act.op, core.ScatterCols) or act in out_set:
+            return None, None
+        H, pieces = st["H"], [result_of(y) for y in act.parents]
+        if any(w != H for w in act.op.widths) or len({prev for (prev, _q) in pieces}) != 1 or pieces[0][0] is None:
+            return None, None
+        if sorted(act.op.offsets) != [H * g for g in range(st["KA"] // H)] or len(pieces) * H != st["KA"]:
+            return None, None
+        return pieces[0][0], [(q, off) for ((_p, q), off) in zip(pieces, act.op.offsets)]
+
+    for node in nodes:
+        if node in steps:
+            st = steps[node]
+            (prev, spec) = act_of(st["product"].parents[0], st)
+            link = None
+            if prev is not None and steps[prev]["sig"] == st["sig"]:
+                state = {}
+                for (k, par) in enumerate(node.parents):
+                    (src, q) = result_of(par)
+                    if k not in st["cols"] and src is prev:
+                        state[k] = q
+                link = (prev, tuple(spec), tuple(sorted(state.items())))
+            st["link"] = link
+
+    done = set()
+    for node in nodes:
+        if node not in steps or node in done or steps[node]["link"] is None:
+            continue
+        how = steps[node]["link"][1:]
+        run = [steps[steps[node]["link"][0]], steps[node]]
+        if run[0]["chain"] in done:
+            continue
+        while True:   # forward while exactly one step follows in the same way
+            after = [n for n in steps if steps[n]["link"] is not None and steps[n]["link"][0] is run[-1]["chain"] and steps[n]["link"][1:] == how]
+            if len(after) != 1:
+                break
+            run.append(steps[after[0]])
+        done.update(s["chain"] for s in run)
+        (spec, state) = (how[0], dict(how[1]))
+        if any(k in run[0]["cols"] or run[0]["chain"].op.in_kinds[k] != 0 for k in state):
+            continue
+        st, op = run[0], run[0]["chain"].op
+        external = [k for k in range(len(op.in_kinds)) if k not in st["cols"] and k not in state]
+        run = _independent_steps(run, external, nodes)
+        per = int(st["bias"]) + len(external) + len(op.out_regs) + 1
+        run = run[:core.Recurrence.MAX_POINTERS // per]
+        if len(run) < 3 or per > core.Recurrence.MAX_PER_STEP or len(state) > 14 or \
+                codegen.recurrence_plan(st["R"], st["H"], st["KA"], st["N"], len(spec)) is None:
+            continue
+        # which results somebody else reads
+        inside = {id(s["chain"]) for s in run} | {id(s["product"]) for s in run}
+        kept, results_of = set(), []
+        scattered = len(spec) > 1 or st["KA"] != st["H"]
+        scatters = []
+        for s in run:
+            parts = defaultdict(list)
+            for c in ([s["chain"]] if not is_tuple(s["chain"]) else children[s["chain"]]):
+                parts[0 if c is s["chain"] else c.op.idx].append(c)
+            results_of.append(parts)
+            scatters.append([n for n in {c for q in parts for part in parts[q] for c in children[part]}
+                             if scattered and isinstance(n.op, core.ScatterCols) and act_of(n, s) == (s["chain"], list(spec))])
+        taken = {id(n) for group in scatters for n in group}
+        for (s, parts) in zip(run, results_of):
+            for q in parts:
+                for part in parts[q]:
+                    if part in out_set or any(id(c) not in inside and id(c) not in taken for c in children[part]):
+                        kept.add(q)
+        if any(part in update_set for parts in results_of for q in parts for part in parts[q]) or any(n in update_set for g in scatters for n in g):
+            continue
+        kept = sorted(kept)
+        rec = core.Recurrence(len(run), st["product"].op.tB, st["bias"], op, st["cols"], state, spec, kept, scattered and any(scatters), st["R"], st["H"],
+                              st["KA"], st["N"])
+        inputs = [st["product"].parents[0]] + list(st["fixed"]) + [st["chain"].parents[k] for k in sorted(state)]
+        results, n_out = [], len(rec.result_shapes())
+        for (i, s) in enumerate(run):
+            inputs += ([s["product"].parents[3]] if st["bias"] else []) + [s["chain"].parents[k] for k in external]
+            for (pos, q) in enumerate(kept):
+                results += [(i * n_out + pos, part) for part in results_of[i][q]]
+            results += [(i * n_out + len(kept), n) for n in scatters[i]]
+        return run, rec, inputs, results
+    return None
+
+
+def _independent_steps(run, external, nodes):
+    """The longest part of `run`, from its first step, whose external operands depend on none of its own steps."""
+    start = {s["chain"]: i for (i, s) in enumerate(run)}
+    position = {}     # node -> the earliest step of the run that it depends on
+    for node in nodes:
+        deps = [position[p] for p in node.parents if p in position]
+        if node in start:
+            deps.append(start[node])
+        if deps:
+            position[node] = min(deps)
+    for (i, s) in enumerate(run):
+        others = [s["chain"].parents[k] for k in external] + ([s["product"].parents[3]] if s["bias"] else [])
+        if i and any(p in position for p in others):
+            return run[:i]
+    return run
+
+
 def fuse_product_sums(outputs, updatetargs, node2shape):
     """z = (X + Repeat(b)) + (Mul22(h, U) + Repeat(c)), the pre-activation of a layer fed by two inputs (an unrolled
     recurrent cell forms it once per layer and time step) -> Mul22BiasAdd(h, U, c, X, b): the three additions run in
@@ -2341,6 +2655,8 @@ def apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape):
             outputs_simple, updatetargs_simple = fuse_flat_index_rows(outputs_simple, updatetargs_simple, node2shape)
         if config["fuse_rows"]:
             outputs_simple, updatetargs_simple = fuse_elementwise(outputs_simple, updatetargs_simple, node2shape, rows=True)
+            if config["batch_summed_products"]:
+                outputs_simple, updatetargs_simple = batch_row_chains(outputs_simple, updatetargs_simple, node2shape)
         outputs_simple, updatetargs_simple = fuse_elementwise(outputs_simple, updatetargs_simple, node2shape)
         if config["fuse_conv_output"]:
             outputs_simple, updatetargs_simple = fuse_conv_output(outputs_simple, updatetargs_simple, node2shape)
@@ -2359,6 +2675,8 @@ def rewrite_for_execution(outputs_simple, updatetargs_simple, updatesrcs, node2s
     """apply_graph_rewrites, then the rewrites that need to know which variables the updates overwrite."""
     config = core.get_config()
     outputs_simple, updatetargs_simple = apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape)
+    if config["fuse_elementwise"] and config["fuse_recurrences"] and config["jit_fused_elementwise"]:
+        outputs_simple, updatetargs_simple = fuse_recurrences(outputs_simple, updatetargs_simple, node2shape)
     # fuse_product_sums switches every use of the products' output stage
     if config["fuse_elementwise"] and config["fuse_product_chains"] and config["fuse_product_sums"]:
         outputs_simple, updatetargs_simple = fuse_product_chains(outputs_simple, updatetargs_simple, updatesrcs, node2shape)

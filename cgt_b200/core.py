@@ -2037,6 +2037,66 @@ class Mul22Chain(Op):
         return "Mul22Chain{%s,%s %r}" % ("T" if self.tA else "N", "T" if self.tB else "N", self.chain)
 
 
+class Recurrence(Op):
+    """`steps` repetitions of (product of the state with one matrix, elementwise chain on it), as one launch.
+
+    Not part of the reference's Op set: compilation.fuse_recurrences forms it from the steps of an unrolled recurrent
+    network, forward or differentiated, that have one and the same chain. Step s computes z = act . op(W), [R, N], with
+    (X_s + abias) + (z + bias) if ``bias``; the chain (``chain``, a FusedElwise over [R, H]) reads columns of z
+    (``z_inputs``: {input: first column}), results of the step before (``state``: {input: result}) and tensors of its own
+    step; ``act_spec`` says which results make up the next step's act: [(result, first column)].
+
+    Inputs: act of the first step, W, (bias, abias), the first step's state inputs in ascending order, then per step
+    (X_s) and the other inputs of the chain. Results per step: those chain results that ``kept`` lists, then act for the
+    next step if ``keep_act``."""
+    available_impls = ("native_gpu",)
+    MAX_PER_STEP, MAX_POINTERS = 32, 3000
+
+    def __init__(self, steps, tB, bias, chain, z_inputs, state, act_spec, kept, keep_act, R, H, KA, N):
+        self.steps, self.tB, self.bias, self.chain = int(steps), bool(tB), bool(bias), chain
+        self.z_inputs, self.state, self.act_spec = dict(z_inputs), dict(state), [tuple(a) for a in act_spec]
+        self.kept, self.keep_act = list(kept), bool(keep_act)
+        self.R, self.H, self.KA, self.N = int(R), int(H), int(KA), int(N)
+        self.external = [k for k in range(len(chain.in_kinds)) if k not in self.z_inputs and k not in self.state]
+
+    def result_shapes(self):
+        return [(self.R, self.H)] * len(self.kept) + [(self.R, self.KA)] * self.keep_act
+
+    def get_diff(self, num_inputs):
+        return [False] * num_inputs
+
+    def shp_apply(self, inputs):
+        one = tuple([cgt.constant(np.array(d, "i8")) for d in shp] for shp in self.result_shapes())
+        return one * self.steps
+
+    def typ_apply(self, input_types):
+        return TupleType(*([TensorType("f4", 2)] * (len(self.result_shapes()) * self.steps)))
+
+    def get_native_compile_info(self, input_types, devtype):
+        from . import codegen
+        need = [self.R * self.N] * self.bias
+        longs = [0] * self.bias
+        for k in self.external:
+            kind = self.chain.in_kinds[k]
+            need.append(1 if kind in (2, 3) else self.R * (self.chain.views[k][1] if kind == 7 else self.H))
+            longs.append(int(kind == 3))
+        outs = [r * c for (r, c) in self.result_shapes()]
+        M = self.MAX_PER_STEP
+        def arr(vals, ctype):
+            return (ctype * M)(*(list(vals) + [0] * (M - len(vals))))
+        return NativeCompileInfo(None, prebuilt="cgtb_op_recurrence", closure_triples=[
+            ("steps", ctypes.c_int, self.steps), ("bias", ctypes.c_int, self.bias), ("n_state", ctypes.c_int, len(self.state)),
+            ("n_ext", ctypes.c_int, len(need)), ("n_out", ctypes.c_int, len(outs)),
+            ("act_size", ctypes.c_long, self.R * self.KA), ("w_size", ctypes.c_long, self.KA * self.N),
+            ("bias_size", ctypes.c_long, self.N), ("state_size", ctypes.c_long, self.R * self.H),
+            ("ext_size", ctypes.c_long * M, arr(need, ctypes.c_long)), ("ext_long", ctypes.c_int * M, arr(longs, ctypes.c_int)),
+            ("out_size", ctypes.c_long * M, arr(outs, ctypes.c_long)),
+            ("launcher", ctypes.c_void_p, codegen.recurrence_launcher(self))])
+
+    def __repr__(self):
+        return "Recurrence{%d x %s %r}" % (self.steps, "N,T" if self.tB else "N,N", self.chain)
+
+
 class BatchedMul22(Op):
     """Per-batch matrix product over the leading axis (cgt/core.py:2231-2288)."""
     available_impls = ("python", "native_cpu", "native_gpu")
@@ -2408,7 +2468,7 @@ _DEFAULTS = dict(
     debug=False, precision="single", backend="native", cache_dir="~/.cgt_b200_cache", enable_inplace_opt=True,
     enable_simplification=True, parallel=False, num_threads=1, force_python_impl=False, debug_cpp=False, verbose=False,
     # additions for this backend
-    devtype="gpu", device_index=0, use_cuda_graphs=True, fuse_elementwise=True, jit_fused_elementwise=True, fuse_conv_dgrad=True, fuse_conv_output=True, fuse_conv_grad_input=True, fuse_conv_implicit=True, fuse_conv_direct=True, fuse_flat_index_rows=True, hoist_filter_splits=True, split_gate_columns=True, fuse_product_sums=True, fuse_product_chains=True, specialise_shapes=True, merge_parameter_updates=True, fuse_rows=True, fuse_slice_sums=True, fuse_slice_views=True, batch_summed_products=True,
+    devtype="gpu", device_index=0, use_cuda_graphs=True, fuse_elementwise=True, jit_fused_elementwise=True, fuse_conv_dgrad=True, fuse_conv_output=True, fuse_conv_grad_input=True, fuse_conv_implicit=True, fuse_conv_direct=True, fuse_flat_index_rows=True, hoist_filter_splits=True, split_gate_columns=True, fuse_product_sums=True, fuse_product_chains=True, fuse_recurrences=True, specialise_shapes=True, merge_parameter_updates=True, fuse_rows=True, fuse_slice_sums=True, fuse_slice_views=True, batch_summed_products=True,
     pad_conv_columns=True, profile=False,
 )
 

@@ -13,6 +13,7 @@
 #include <cstring>
 #include <limits>
 #include <type_traits>
+#include <vector>
 
 using namespace cgtb;
 
@@ -385,6 +386,49 @@ OP_BYREF(cgtb_op_mul22_bias_add) {
   }
   cgtb_sgemm_bias_add(cl->tA, cl->tB, M, N, K, (const float*)A->data(), lda, (const float*)B->data(), ldb, (const float*)bias->data(),
                       (const float*)add->data(), N, (const float*)abias->data(), (float*)C->data(), ldc);
+}
+// Recurrence: the steps of an unrolled recurrent network in one launch of a generated kernel. reads = act of the first
+// step, W, (bias, abias), n_state state arrays, then n_ext arrays per step; results: n_out arrays per step.
+struct RecurrenceClosure {
+  int steps, bias, n_state, n_ext, n_out;
+  long act_size, w_size, bias_size, state_size, ext_size[32];
+  int ext_long[32];
+  long out_size[32];
+  void* launcher;
+};
+typedef int (*RecurrenceLauncher)(int steps, const void* const* fixed, const void* const* per_step, void* stream);
+OP_BYREF(cgtb_op_recurrence) {
+  const RecurrenceClosure* cl = (const RecurrenceClosure*)cl0;
+  if (!cl->launcher) { fail("Recurrence: its kernel was not generated"); return; }
+  const int n_fixed = 2 + 2 * cl->bias + cl->n_state, per = cl->n_ext + cl->n_out;
+  if (n_fixed > 20 || cl->n_ext > 32 || cl->n_out > 32) { fail("Recurrence: too many operands"); return; }
+  const void* fixed[20];
+  for (int k = 0; k < n_fixed; ++k) {
+    cgtArray* x = ARR(reads[k]);
+    const long want = k == 0 ? cl->act_size : k == 1 ? cl->w_size : k < 2 + 2 * cl->bias ? cl->bias_size : cl->state_size;
+    if (!on_gpu(x) || x->dtype() != cgt_f4 || x->size() != want) { fail("Recurrence: operand %d is not a float32 GPU array of %ld elements", k, want); return; }
+    fixed[k] = x->data();
+  }
+  static thread_local std::vector<const void*> ptrs;
+  ptrs.resize((size_t)cl->steps * per);
+  cgtTuple* results = (cgtTuple*)write0;
+  for (int s = 0; s < cl->steps; ++s) {
+    for (int k = 0; k < cl->n_ext; ++k) {
+      cgtArray* x = ARR(reads[n_fixed + s * cl->n_ext + k]);
+      if (!on_gpu(x) || x->dtype() != (cl->ext_long[k] ? cgt_i8 : cgt_f4) || x->size() != cl->ext_size[k]) {
+        fail("Recurrence: operand %d of step %d is not a GPU array of %ld elements of its type", k, s, cl->ext_size[k]);
+        return;
+      }
+      ptrs[(size_t)s * per + k] = x->data();
+    }
+    for (int q = 0; q < cl->n_out; ++q) {
+      cgtArray* w = ARR(results->getitem(s * cl->n_out + q));
+      if (!on_gpu(w) || w->dtype() != cgt_f4 || w->size() != cl->out_size[q]) { fail("Recurrence: result %d of step %d has the wrong size", q, s); return; }
+      ptrs[(size_t)s * per + cl->n_ext + q] = w->data();
+    }
+  }
+  if (((RecurrenceLauncher)cl->launcher)(cl->steps, fixed, ptrs.data(), (void*)rt().stream)) { cudaGetLastError(); fail("Recurrence: launch failed"); return; }
+  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
 }
 struct BMul22Closure { bool tA; bool tB; };
 OP_BYREF(cgtb_op_batched_mul22) {

@@ -576,3 +576,35 @@ def test_copies_per_shape_do_not_thrash(monkeypatch, n_shapes):
         assert len(compiled) <= f.MOST + n_shapes * 6
     monkeypatch.setattr(compilation._SpecialisedByShape, "_room", staticmethod(lambda: False))
     assert f(np.zeros((99, 3), "f4")) == "general" and f([[1.0, 2.0]]) == "general"
+
+
+def _gpu_ops(cfg):
+    eg = compilation.execution_graph(cfg.inputs, [cfg.loss] + list(cfg.extra_outputs), cfg.updates, [])[0]
+    return [i.op for i in eg.instrs if getattr(i, "op", None) is not None]
+
+
+@pytest.mark.parametrize("T,B,V,H,L", [(8, 64, 65, 128, 2), (15, 33, 47, 90, 1), (6, 24, 40, 100, 2)])
+def test_steps_of_an_unrolled_network_are_grouped(monkeypatch, T, B, V, H, L):
+    from cgt_b200 import codegen
+    monkeypatch.setattr(codegen, "recurrence_launcher", lambda op: 1)
+    ops = _gpu_ops(configs.build_lstm(vocab=V, hidden=H, n_layers=L, seq_len=T, batch=B))
+    recs = [op for op in ops if isinstance(op, core.Recurrence)]
+    assert [r.steps for r in recs] == [T - 2] * (2 * L)   # the first and the last step have chains of their own
+    assert sorted(r.bias for r in recs) == [False] * L + [True] * L
+    assert sum(isinstance(op, core.FusedRows) for op in ops) == 1
+    monkeypatch.setattr(codegen, "recurrence_launcher", lambda op: None)   # no compiler: the steps stay as they are
+    assert not any(isinstance(op, core.Recurrence) for op in _gpu_ops(configs.build_lstm(vocab=V, hidden=H, n_layers=L, seq_len=T, batch=B)))
+
+
+def test_recurrence_plans_cover_their_extents():
+    from cgt_b200 import codegen
+    for R in (1, 2, 7, 33, 64, 129, 256):
+        for H in list(range(1, 140)) + [160, 200, 256, 300]:
+            for NG in (1, 2, 3, 4):
+                for (KA, N) in ((H, NG * H), (NG * H, H)):
+                    p = codegen.recurrence_plan(R, H, KA, N, 1)
+                    if p is None:
+                        continue
+                    assert p["C"] * p["UH"] >= H > (p["C"] - 1) * p["UH"] and p["NC"] == p["UH"] * (N // H)
+                    assert p["KG"] * p["KT"] >= KA > (p["KG"] - 1) * p["KT"] and p["KT"] % 4 == 0 and p["KG"] * p["NC"] <= 256
+                    assert p["RB"] * p["UH"] <= 256 and 4 * (2 * p["RB"] * p["KG"] * p["KT"] + p["KG"] * p["RB"] * p["NC"]) <= 48 * 1024
