@@ -2655,8 +2655,6 @@ def apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape):
             outputs_simple, updatetargs_simple = fuse_flat_index_rows(outputs_simple, updatetargs_simple, node2shape)
         if config["fuse_rows"]:
             outputs_simple, updatetargs_simple = fuse_elementwise(outputs_simple, updatetargs_simple, node2shape, rows=True)
-            if config["batch_summed_products"]:
-                outputs_simple, updatetargs_simple = batch_row_chains(outputs_simple, updatetargs_simple, node2shape)
         outputs_simple, updatetargs_simple = fuse_elementwise(outputs_simple, updatetargs_simple, node2shape)
         if config["fuse_conv_output"]:
             outputs_simple, updatetargs_simple = fuse_conv_output(outputs_simple, updatetargs_simple, node2shape)
@@ -2672,9 +2670,11 @@ def apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape):
 
 
 def rewrite_for_execution(outputs_simple, updatetargs_simple, updatesrcs, node2shape):
-    """apply_graph_rewrites, then the rewrites that need to know which variables the updates overwrite."""
+    """apply_graph_rewrites, then the rewrites over the finished chains: over time steps, and into the products."""
     config = core.get_config()
     outputs_simple, updatetargs_simple = apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape)
+    if config["fuse_elementwise"] and config["fuse_rows"] and config["batch_summed_products"]:
+        outputs_simple, updatetargs_simple = batch_row_chains(outputs_simple, updatetargs_simple, node2shape)
     if config["fuse_elementwise"] and config["fuse_recurrences"] and config["jit_fused_elementwise"]:
         outputs_simple, updatetargs_simple = fuse_recurrences(outputs_simple, updatetargs_simple, node2shape)
     # fuse_product_sums switches every use of the products' output stage
