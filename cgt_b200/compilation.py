@@ -2675,7 +2675,8 @@ def rewrite_for_execution(outputs_simple, updatetargs_simple, updatesrcs, node2s
     outputs_simple, updatetargs_simple = apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape)
     if config["fuse_elementwise"] and config["fuse_rows"] and config["batch_summed_products"]:
         outputs_simple, updatetargs_simple = batch_row_chains(outputs_simple, updatetargs_simple, node2shape)
-    if config["fuse_elementwise"] and config["fuse_recurrences"] and config["jit_fused_elementwise"]:
+    # fuse_rows switches every chain that adds up in another order than the separate Ops
+    if config["fuse_elementwise"] and config["fuse_rows"] and config["fuse_recurrences"] and config["jit_fused_elementwise"]:
         outputs_simple, updatetargs_simple = fuse_recurrences(outputs_simple, updatetargs_simple, node2shape)
     # fuse_product_sums switches every use of the products' output stage
     if config["fuse_elementwise"] and config["fuse_product_chains"] and config["fuse_product_sums"]:
