@@ -861,6 +861,105 @@ def batch_row_chains(outputs, updatetargs, node2shape):
     return _rewire(outputs, updatetargs, replace)
 
 
+def fuse_square_sums(outputs, updatetargs, node2shape):
+    """Sum(square(x)) over all axes of several float32 arrays, none of which needs another's sum -> SumSquares, one launch
+    for all of them. Arrays of up to 2^20 elements: a larger one keeps more blocks busy than the eight it has here."""
+    all_out = list(outputs) + list(updatetargs)
+    nodes = core.topsorted(all_out)
+    children = defaultdict(list)
+    for node in nodes:
+        for par in node.parents:
+            children[par].append(node)
+    out_set = set(all_out)
+    found, reached = [], set()
+    for node in nodes:
+        if any(p in reached for p in node.parents):
+            reached.add(node)
+        if node in out_set or node.is_input() or type(node.op) is not core.Sum or node.dtype != "f4" or len(found) == core.SumSquares.MOST:
+            continue
+        sq = node.parents[0]
+        if sq.is_input() or not isinstance(sq.op, core.ElwiseUnary) or sq.op.opname != "square" or sq in out_set or children[sq] != [node]:
+            continue
+        (x, shp) = (sq.parents[0], _static_shape(node2shape[sq]))
+        if x.dtype != "f4" or shp is None or len(node.op.axes) != len(shp) or not 1 <= np.prod(shp, dtype=np.int64) <= 1 << 20 or x in reached:
+            continue
+        found.append((node, x))
+        reached.add(node)
+    if len(found) < 2:
+        return list(outputs), list(updatetargs)
+    new = core.Result(core.SumSquares([node.ndim for (node, _x) in found]), [x for (_node, x) in found])
+    node2shape[new] = tuple(list(node2shape[node]) for (node, _x) in found)
+    replace = {}
+    for (i, (node, _x)) in enumerate(found):
+        part = core.Result(core.TupleIndex(i), [new])
+        node2shape[part] = node2shape[node]
+        part.props.update(node.props)
+        replace[node] = part
+    return _rewire(outputs, updatetargs, replace)
+
+
+def split_shared_updates(outputs, updatetargs):
+    """An elementwise operation that only several updates read (lr * g of a gradient that two parameters have in common)
+    is repeated for each of them: every update is a chain of its own then and all of them one launch. Returns {copy:
+    the node it repeats}."""
+    nodes = core.topsorted(list(outputs) + list(updatetargs))
+    children = defaultdict(list)
+    for node in nodes:
+        for par in node.parents:
+            children[par].append(node)
+    (out_set, targets) = (set(outputs), set(updatetargs))
+    private = set(targets)     # update targets and what only they read
+    for node in reversed(nodes):
+        if _fusable(node) and node not in out_set and children[node] and all(c in private for c in children[node]):
+            private.add(node)
+    copies = {}
+
+    def copy_of(node, first, shared=False):
+        shared = shared or (not first and len(children[node]) > 1)
+        parents = [copy_of(p, False, shared) if p in private and p not in targets else p for p in node.parents]
+        if first:
+            node.parents[:] = parents
+            return node
+        if not shared and parents == list(node.parents):
+            return node
+        new = core.Result(node.op, parents)
+        new.props.update(node.props)
+        copies[new] = node
+        return new
+    for t in updatetargs:
+        if not t.is_input() and _fusable(t) and not any(c in targets for c in children[t]):
+            copy_of(t, True)
+    return copies
+
+
+def delay_host_arithmetic(eg):
+    """Instruction-list pass: host instructions on values that come from the device move behind the device work that does
+    not need them, up to the first instruction that does. Every change from device to host and back ends a span with a
+    wait: the ten sums of squares of a clipped gradient are downloaded together instead of one after the other."""
+    delayed, fresh, reads_of, writes_of, out, written = [], set(), set(), set(), [], set()
+    for ins in eg.instrs:
+        read_locs = getattr(ins, "read_locs", [])
+        reads, w = {r.index for r in read_locs}, ins.write_loc.index
+        on_host = ins.write_loc.devtype == "cpu" and all(r.devtype == "cpu" for r in read_locs)
+        # an Alloc gives a location its memory, whatever writes it again works in place
+        in_place = w in written and ins.write_loc.devtype == "cpu"
+        if not isinstance(ins, Alloc):
+            written.add(w)
+        if on_host and isinstance(ins, (ReturnByRef, ReturnByVal)) and reads & (fresh | writes_of) and not in_place and w not in reads_of:
+            delayed.append(ins)
+            reads_of |= reads
+            writes_of.add(w)
+            continue
+        if reads & writes_of or w in writes_of or w in reads_of or in_place:
+            out += delayed
+            (delayed, fresh, reads_of, writes_of) = ([], set(), set(), set())
+        out.append(ins)
+        if ins.write_loc.devtype == "cpu" and not on_host:
+            fresh.add(w)
+    eg.instrs = out + delayed
+    return eg
+
+
 def fuse_recurrences(outputs, updatetargs, node2shape):
     """Consecutive steps of an unrolled recurrent network, forward or differentiated -> Recurrence, one launch.
 
@@ -2650,6 +2749,9 @@ def apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape):
         outputs_simple, updatetargs_simple = batch_scalar_sums(outputs_simple, updatetargs_simple, node2shape)
     if config["fuse_product_sums"]:    # after the batching: the products over all time steps are views by now
         outputs_simple, updatetargs_simple = fuse_product_sums(outputs_simple, updatetargs_simple, node2shape)
+    if config["fuse_elementwise"] and config["merge_parameter_updates"]:
+        for (new, old) in split_shared_updates(outputs_simple, updatetargs_simple).items():
+            node2shape[new] = node2shape[old]
     if config["fuse_elementwise"]:
         if config["fuse_rows"] and config["fuse_flat_index_rows"]:
             outputs_simple, updatetargs_simple = fuse_flat_index_rows(outputs_simple, updatetargs_simple, node2shape)
@@ -2675,7 +2777,9 @@ def rewrite_for_execution(outputs_simple, updatetargs_simple, updatesrcs, node2s
     outputs_simple, updatetargs_simple = apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape)
     if config["fuse_elementwise"] and config["fuse_rows"] and config["batch_summed_products"]:
         outputs_simple, updatetargs_simple = batch_row_chains(outputs_simple, updatetargs_simple, node2shape)
-    # fuse_rows switches every chain that adds up in another order than the separate Ops
+    # fuse_rows switches everything that adds up in another order than the separate Ops
+    if config["fuse_square_sums"] and config["fuse_rows"]:
+        outputs_simple, updatetargs_simple = fuse_square_sums(outputs_simple, updatetargs_simple, node2shape)
     if config["fuse_elementwise"] and config["fuse_rows"] and config["fuse_recurrences"] and config["jit_fused_elementwise"]:
         outputs_simple, updatetargs_simple = fuse_recurrences(outputs_simple, updatetargs_simple, node2shape)
     # fuse_product_sums switches every use of the products' output stage
@@ -2709,6 +2813,8 @@ def execution_graph(inputs, outputs, updates, givens):
     eg, node2memloc = create_execution_graph(inputs, nodes_sorted, node2shape, node2memowner, node2dev, once_nodes)
     if config["merge_parameter_updates"] and updates_simple:
         merge_parameter_updates(eg, set(node2memloc[t].index for t in updatetargs_simple))
+    if config["delay_host_arithmetic"]:
+        delay_host_arithmetic(eg)
 
     if config["verbose"]:
         sys.stderr.write("begin\n" + "\n".join("%i.) \t%r" % (i, instr) for (i, instr) in enumerate(eg.instrs)) + "\nend\n")

@@ -2000,6 +2000,32 @@ class Mul22BiasAdd(Op):
         return "Mul22BiasAdd{%s,%s}" % ("T" if self.tA else "N", "T" if self.tB else "N")
 
 
+class SumSquares(Op):
+    """(x_0, x_1, ...) -> the sum of squares of each, with all axes kept at extent 1. Not part of the reference's Op set:
+    compilation.fuse_square_sums forms it from Sum(square(x)) of several arrays (the global norm of all gradients)."""
+    available_impls = ("native_gpu",)
+    MOST = 32
+
+    def __init__(self, ndims):
+        self.ndims = tuple(ndims)
+        assert 1 <= len(self.ndims) <= self.MOST
+
+    def get_diff(self, num_inputs):
+        return [False] * num_inputs
+
+    def shp_apply(self, inputs):
+        return tuple([cgt.constant(np.array(1, "i8"))] * n for n in self.ndims)
+
+    def typ_apply(self, input_types):
+        return TupleType(*[TensorType("f4", n) for n in self.ndims])
+
+    def get_native_compile_info(self, input_types, devtype):
+        return NativeCompileInfo(None, prebuilt="cgtb_op_sum_squares", closure_triples=[("k", ctypes.c_int, len(self.ndims))])
+
+    def __repr__(self):
+        return "SumSquares{%d}" % len(self.ndims)
+
+
 class Mul22Chain(Op):
     """(A, B, other inputs of the chain) -> results of an elementwise chain on op(A).op(B) [M, N] and those inputs.
 
@@ -2468,7 +2494,7 @@ _DEFAULTS = dict(
     debug=False, precision="single", backend="native", cache_dir="~/.cgt_b200_cache", enable_inplace_opt=True,
     enable_simplification=True, parallel=False, num_threads=1, force_python_impl=False, debug_cpp=False, verbose=False,
     # additions for this backend
-    devtype="gpu", device_index=0, use_cuda_graphs=True, fuse_elementwise=True, jit_fused_elementwise=True, fuse_conv_dgrad=True, fuse_conv_output=True, fuse_conv_grad_input=True, fuse_conv_implicit=True, fuse_conv_direct=True, fuse_flat_index_rows=True, hoist_filter_splits=True, split_gate_columns=True, fuse_product_sums=True, fuse_product_chains=True, fuse_recurrences=True, specialise_shapes=True, merge_parameter_updates=True, fuse_rows=True, fuse_slice_sums=True, fuse_slice_views=True, batch_summed_products=True,
+    devtype="gpu", device_index=0, use_cuda_graphs=True, fuse_elementwise=True, jit_fused_elementwise=True, fuse_conv_dgrad=True, fuse_conv_output=True, fuse_conv_grad_input=True, fuse_conv_implicit=True, fuse_conv_direct=True, fuse_flat_index_rows=True, hoist_filter_splits=True, split_gate_columns=True, fuse_product_sums=True, fuse_product_chains=True, fuse_recurrences=True, fuse_square_sums=True, delay_host_arithmetic=True, specialise_shapes=True, merge_parameter_updates=True, fuse_rows=True, fuse_slice_sums=True, fuse_slice_views=True, batch_summed_products=True,
     pad_conv_columns=True, profile=False,
 )
 

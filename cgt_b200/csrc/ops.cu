@@ -710,6 +710,24 @@ OP_BYREF(cgtb_op_reduce) {
   fail("Sum/Max: operands must be on the GPU");
 }
 
+// SumSquares: (x_0, x_1, ...) -> one sum of squares each
+struct SumSquaresClosure { int k; };
+OP_BYREF(cgtb_op_sum_squares) {
+  const int k = ((SumSquaresClosure*)cl0)->k;
+  if (k < 1 || k > CGTB_SUM_SQUARES_MAX) { fail("SumSquares: between 1 and %d arrays", CGTB_SUM_SQUARES_MAX); return; }
+  const void* in[CGTB_SUM_SQUARES_MAX];
+  void* out[CGTB_SUM_SQUARES_MAX];
+  long n[CGTB_SUM_SQUARES_MAX];
+  for (int t = 0; t < k; ++t) {
+    cgtArray *x = ARR(reads[t]), *w = ARR(((cgtTuple*)write0)->getitem(t));
+    if (!all_gpu({x, w}) || x->dtype() != cgt_f4 || w->dtype() != cgt_f4 || w->size() != 1) { fail("SumSquares: operands must be float32 GPU arrays"); return; }
+    in[t] = x->data();
+    out[t] = w->data();
+    n[t] = x->size();
+  }
+  cgtb_sum_squares(k, n, in, out);
+}
+
 // ------------------------------------------------------------------------------------------------
 // Repeat / Transpose / slices / flat indices / Concatenate / Fill / constants
 // ------------------------------------------------------------------------------------------------

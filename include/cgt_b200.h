@@ -408,6 +408,11 @@ int cgtb_comm_rank(void);
 int cgtb_comm_check(void);   /* non-zero when NCCL reported an asynchronous error */
 int cgtb_comm_abort(void);
 int cgtb_comm_destroy(void);
+/* Sums of squares of k float32 device arrays, out[t] a single float: one launch. No counterpart in the reference, which
+ * squares and sums each array by itself. */
+#define CGTB_SUM_SQUARES_MAX 32
+int cgtb_sum_squares(int k, const long* n, const void* const* in, void* const* out);
+
 /* out[i] = sum over ranks of in[i] for n float buffers, one NCCL group on the runtime stream */
 int cgtb_allreduce_sum(int dtype, int n, const void* const* in, void* const* out, const long* counts);
 

@@ -78,3 +78,34 @@ def test_cell_with_results_handed_out(rt, B, H):
 def test_feedback_by_another_way_is_not_grouped(rt):
     out = _both_ways(_cells(6, 40, 48, True), 4)
     _close(out, 96, 6)
+
+
+@pytest.mark.parametrize("dtype", ["f4", "f8"])
+def test_column_sums_over_a_cluster_of_blocks(rt, dtype):
+    """[R, K] over R: rows around those at which two, four and eight blocks share a column, with and without a remainder."""
+    from cgt_b200 import runtime
+    rs = np.random.RandomState(5)
+    for (R, K) in [(255, 33), (256, 1), (257, 70), (511, 32), (512, 31), (513, 512), (1023, 40), (1024, 64), (1025, 129), (2048, 2400), (3200, 512), (4096, 5)]:
+        a = rs.randn(R, K).astype(dtype)
+        with cgt.scoped_update_config(precision="single" if dtype == "f4" else "double"):
+            x = cgt.matrix("x")
+            f = cgt.function([x], [cgt.sum(x, axis=0), cgt.max(x, axis=0)])
+        (total, top) = f(runtime.device_array(a))
+        # any order of R additions is off by at most R * eps * sum |a|
+        assert (np.abs(total.reshape(-1) - a.astype("f8").sum(0)) <= R * np.finfo(dtype).eps * np.abs(a).sum(0)).all(), (R, K)
+        assert np.array_equal(top.reshape(-1), a.max(0))
+
+
+def test_sums_of_squares_of_many_arrays(rt):
+    """Every remainder of the 16-byte loads, one element, ragged views, more arrays than one launch takes."""
+    shapes = [(1, 1), (3, 1), (1, 5), (65, 512), (7, 4096), (1, 4097), (128, 33), (1024, 1024)] + [(i + 1, 3) for i in range(30)]
+    xs = [cgt.matrix("x%d" % i, fixed_shape=s) for (i, s) in enumerate(shapes)]
+    for on in (False, True):
+        with cgt.scoped_update_config(fuse_square_sums=on):
+            f = cgt.function(xs, [cgt.square(x).sum() * 1.0 for x in xs])
+        assert any(isinstance(getattr(i, "op", None), core.SumSquares) for i in f.eg.instrs) == on
+        for call in range(3):
+            vals = [np.random.RandomState(call).randn(*s).astype("f4") for s in shapes]
+            for (v, got) in zip(vals, f(*vals)):
+                want = np.square(v.astype("f8")).sum()
+                assert abs(got - want) <= v.size * np.finfo("f4").eps * want
