@@ -748,7 +748,7 @@ def batch_row_chains(outputs, updatetargs, node2shape):
     """FusedRows nodes of one program whose matrices are the consecutive leading slices of whole arrays, whose other
     operands are the same and none of which needs another's result (the softmax and its pullback at every time step of
     an unrolled network) -> ONE FusedRows over the whole arrays, every original result a LeadingSlice view of its result.
-    Rows are independent of each other, so no bit changes. Fifty launches on [64, 65] take 150 us, the one 4 us."""
+    Rows are independent of each other, so no bit changes. Fifty launches on [64, 65] are one."""
     all_out = list(outputs) + list(updatetargs)
     nodes = core.topsorted(all_out)
     children = defaultdict(list)
@@ -968,7 +968,7 @@ def fuse_recurrences(outputs, updatetargs, node2shape):
     belong together while chain, matrix and the way in which one feeds the next are the same; the first and the last step
     of a network usually differ and stay as they are. A step whose other operands depend on an earlier step of the same
     group by another way starts a new group. Products and chains that run as they are take two to three launches of 3 us
-    per step, half of it latency; a step of the one launch takes about 0.7 us."""
+    per step, half of it latency; 48 steps of 64 x 128 units in the one launch took 72 us, 1.5 us each."""
     from . import codegen
     refused = set()
     while True:
@@ -1103,7 +1103,7 @@ def _find_recurrence(nodes, children, out_set, update_set, node2shape, refused):
         run = _independent_steps(run, external, nodes)
         per = int(st["bias"]) + len(external) + len(op.out_regs) + 1
         run = run[:core.Recurrence.MAX_POINTERS // per]
-        if len(run) < 3 or per > core.Recurrence.MAX_PER_STEP or len(state) > 14 or \
+        if len(run) < core.Recurrence.LEAST or per > core.Recurrence.MAX_PER_STEP or len(state) > 14 or \
                 codegen.recurrence_plan(st["R"], st["H"], st["KA"], st["N"], len(spec)) is None:
             continue
         # which results somebody else reads

@@ -2076,7 +2076,9 @@ class Recurrence(Op):
     (X_s) and the other inputs of the chain. Results per step: those chain results that ``kept`` lists, then act for the
     next step if ``keep_act``."""
     available_impls = ("native_gpu",)
-    MAX_PER_STEP, MAX_POINTERS = 32, 3000
+    # LEAST: a kernel of its own is compiled for the group and its launch fills the registers with W; a few steps keep
+    # their separate launches, and their bits
+    MAX_PER_STEP, MAX_POINTERS, LEAST = 32, 3000, 5
 
     def __init__(self, steps, tB, bias, chain, z_inputs, state, act_spec, kept, keep_act, R, H, KA, N):
         self.steps, self.tB, self.bias, self.chain = int(steps), bool(tB), bool(bias), chain

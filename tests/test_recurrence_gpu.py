@@ -33,15 +33,15 @@ def _close(out, K, T):
         assert np.linalg.norm(a.astype("f8") - b) <= bound * max(np.linalg.norm(a), 1e-3)
 
 
-@pytest.mark.parametrize("T,B,V,H,L", [(5, 64, 65, 128, 2), (6, 1, 30, 32, 1), (7, 64, 40, 32, 1), (5, 33, 47, 90, 1), (9, 17, 31, 50, 2),
-                                       (6, 129, 35, 64, 1), (5, 7, 33, 101, 1), (5, 31, 30, 129, 1), (50, 8, 30, 100, 1)])
+@pytest.mark.parametrize("T,B,V,H,L", [(7, 64, 65, 128, 2), (8, 1, 30, 32, 1), (7, 64, 40, 32, 1), (7, 33, 47, 90, 1), (9, 17, 31, 50, 2),
+                                       (8, 129, 35, 64, 1), (7, 7, 33, 101, 1), (7, 31, 30, 129, 1), (50, 8, 30, 100, 1)])
 def test_lstm_training_step(rt, T, B, V, H, L):
     def build():
         cfg = configs.build_lstm(vocab=V, hidden=H, n_layers=L, seq_len=T, batch=B)
         return cfg.compile(), [v for (v, _new) in cfg.updates], cfg.batch_fn
     out = _both_ways(build, 4)
     (got, recs) = out[True]
-    assert recs and all(r.steps >= 3 for r in recs)
+    assert recs and all(r.steps >= core.Recurrence.LEAST for r in recs)
     _close(out, 4 * H, T)
 
 
@@ -76,8 +76,8 @@ def test_cell_with_results_handed_out(rt, B, H):
 
 
 def test_feedback_by_another_way_is_not_grouped(rt):
-    out = _both_ways(_cells(6, 40, 48, True), 4)
-    _close(out, 96, 6)
+    out = _both_ways(_cells(9, 40, 48, True), 4)
+    _close(out, 96, 9)
 
 
 @pytest.mark.parametrize("dtype", ["f4", "f8"])
