@@ -351,7 +351,8 @@ def recurrence_source(op):
     """CUDA source of the kernel for one Recurrence (plan: recurrence_plan). One step: every thread multiplies its KT
     weights (registers) with the rows' act (shared memory, broadcast reads), the K groups' partial sums meet in shared
     memory, one thread per (row, unit) adds them in order, runs the chain and writes its part of the next act into the
-    shared memory of all blocks of the cluster; a cluster barrier ends the step. The act is double-buffered, so one barrier
+    shared memory of all blocks of the cluster; a cluster barrier ends the step, and what goes to global memory is written
+    between a block's arrival there and its wait. The act is double-buffered, so one barrier
     per step is enough; the chain's other operands are loaded a step ahead.
 
     Bound by that serial chain, not by operations: the FMAs of a step (2 rows x 128 columns x 128 per block) take about
@@ -379,10 +380,14 @@ def recurrence_source(op):
          'struct Job { const void* fixed[20]; int steps; const void* p[kPointers]; };',
          '// Warps come here from divergent code: they gather first, and every thread arrives for itself (no .aligned). Reached',
          '// without any condition in every step, the last one included: under one (s + 1 < steps, which the chain tests as well)',
-         '// the two halves of a warp may take different ways to it.',
-         '__device__ __forceinline__ void step_barrier() {',
+         '// the two halves of a warp may take different ways to it. The results go to global memory between arrival and wait:',
+         '// before the arrival, its release would wait for them.',
+         '__device__ __forceinline__ void step_arrive() {',
          '  __syncwarp();',
-         '  if (C > 1) asm volatile("barrier.cluster.arrive.release;\\n\\tbarrier.cluster.wait.acquire;" ::: "memory");',
+         '  if (C > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");', '}',
+         '__device__ __forceinline__ void step_wait() {',
+         '  __syncwarp();',
+         '  if (C > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");',
          '  else __syncthreads();', '}',
          '__device__ __forceinline__ void store_peer(float* own, int block, float v) {',
          '  if (C == 1) { *own = v; return; }',
@@ -420,7 +425,7 @@ def recurrence_source(op):
     L += ['  float %s;' % ", ".join("%s = 0.0f, next_%s = 0.0f" % (r, r) for r in regs)] if regs else []
     fetch = ['      next_%s = %s;' % (r, ld) for (r, ld) in zip(regs, loads)]
     L += ['  if (live) {', '    const void* const* q = a.p;', '    (void)q;'] + fetch + ['  }',
-          '  step_barrier();',
+          '  step_arrive();', '  step_wait();',
           '  for (int s = 0; s < a.steps; ++s) {',
           '    const void* const* now = a.p + s * PER;', '    (void)now;']
     L += ['    %s = next_%s;' % (r, r) for r in regs]
@@ -442,8 +447,9 @@ def recurrence_source(op):
           '#pragma unroll',
           '      for (int r = 0; r < RB; ++r) part[kg][r][col] = sum[r];',
           '    }',
-          '    __syncthreads();',
-          '    if (live) {']
+          '    __syncthreads();']
+    stored = sorted(set(op.kept) | {q for (q, _off) in op.act_spec} | {op.state[k] for k in states})
+    L += ['    float %s;' % ", ".join("o%d = 0.0f" % q for q in stored), '    if (live) {']
     for g in range(p["NG"]):
         L += ['      float z%d = part[0][rr][%d + u];' % (g, g * p["UH"]), '#pragma unroll',
               '      for (int k = 1; k < KG; ++k) z%d += part[k][rr][%d + u];' % (g, g * p["UH"])]
@@ -455,19 +461,19 @@ def recurrence_source(op):
     for (i, (arity, code, x, y)) in enumerate(chain.program):
         L.append('      const float r%d = %s;' % (n_in + i, "unary_apply<float, float>(%d, r%d)" % (code, x) if arity == 1 else
                                                   "binary_apply<float, float, float>(%d, r%d, r%d)" % (code, x, y)))
-    at = ext0 + len(op.external)
-    for (pos, q) in enumerate(op.kept):
-        L.append('      ((float*)now[%d])[row * H + j] = r%d;' % (at + pos, chain.out_regs[q]))
-    if op.keep_act:
-        for (q, off) in op.act_spec:
-            L.append('      ((float*)now[%d])[row * KA + %d + j] = r%d;' % (at + len(op.kept), off, chain.out_regs[q]))
-    for k in states:
-        L.append('      t%d = r%d;' % (k, chain.out_regs[op.state[k]]))
+    L += ['      o%d = r%d;' % (q, chain.out_regs[q]) for q in stored]
+    L += ['      t%d = o%d;' % (k, op.state[k]) for k in states]
     L += ['      float* dst = &act[(s + 1) & 1][rr][j];',
           '#pragma unroll', '      for (int c = 0; c < C; ++c) {']
-    L += ['        store_peer(dst + %d, c, r%d);' % (off, chain.out_regs[q]) for (q, off) in op.act_spec]
-    L += ['      }', '    }',
-          '    step_barrier();',
+    L += ['        store_peer(dst + %d, c, o%d);' % (off, q) for (q, off) in op.act_spec]
+    L += ['      }', '    }', '    step_arrive();', '    if (live) {']
+    at = ext0 + len(op.external)
+    for (pos, q) in enumerate(op.kept):
+        L.append('      ((float*)now[%d])[row * H + j] = o%d;' % (at + pos, q))
+    if op.keep_act:
+        for (q, off) in op.act_spec:
+            L.append('      ((float*)now[%d])[row * KA + %d + j] = o%d;' % (at + len(op.kept), off, q))
+    L += ['    }', '    step_wait();',
           '  }', '}', '}  // namespace',
           'extern "C" __attribute__((visibility("default"))) int cgtb_recurrence_launch(int steps, const void* const* fixed,',
           '    const void* const* per_step, void* stream) {',
