@@ -267,6 +267,26 @@ def _foldable_repeat(node):
     return all(b - a == 1 for (a, b) in zip(kept[:-1], kept[1:]))
 
 
+def variables_seen(node):
+    """The shared variables whose memory `node` is or views."""
+    (found, stack) = (set(), [node])
+    while stack:
+        n = stack.pop()
+        if n.is_data():
+            found.add(n)
+        elif not n.is_input() and n.op.return_type == "byval" and not isinstance(n.op, core.Size):
+            stack.extend(n.parents)
+    return found
+
+
+def variables_read(node):
+    """The shared variables whose memory the operation of `node` reads; operands of which only the extents count are none."""
+    if node.is_input():
+        return set()
+    skip = _meta_inputs(node.op, len(node.parents))
+    return set().union(*[variables_seen(par) for (pos, par) in enumerate(node.parents) if pos not in skip])
+
+
 def view_leading_slices(outputs, updatetargs, node2shape):
     """GetSli along axis 0 with step 1 and constant bounds -> LeadingSlice: the rows of a C-contiguous array are contiguous,
     so the slice is a view at an offset instead of a copy kernel. Only where the source cannot change under the view:
@@ -898,16 +918,18 @@ def fuse_square_sums(outputs, updatetargs, node2shape):
     return _rewire(outputs, updatetargs, replace)
 
 
-def split_shared_updates(outputs, updatetargs):
+def split_shared_updates(outputs, updatetargs, updatesrcs=()):
     """An elementwise operation that only several updates read (lr * g of a gradient that two parameters have in common)
     is repeated for each of them: every update is a chain of its own then and all of them one launch. Returns {copy:
-    the node it repeats}."""
+    the node it repeats}. An operation that reads a variable which this step overwrites is not repeated (mu * v of a
+    velocity that Nesterov's step reads before and after its update): a copy would run where its chain runs, which may be
+    after that variable's update."""
     nodes = core.topsorted(list(outputs) + list(updatetargs))
     children = defaultdict(list)
     for node in nodes:
         for par in node.parents:
             children[par].append(node)
-    (out_set, targets) = (set(outputs), set(updatetargs))
+    (out_set, targets, overwritten) = (set(outputs), set(updatetargs), set(updatesrcs))
     private = set(targets)     # update targets and what only they read
     for node in reversed(nodes):
         if _fusable(node) and node not in out_set and children[node] and all(c in private for c in children[node]):
@@ -916,6 +938,8 @@ def split_shared_updates(outputs, updatetargs):
 
     def copy_of(node, first, shared=False):
         shared = shared or (not first and len(children[node]) > 1)
+        if shared and variables_read(node) & overwritten:
+            return node
         parents = [copy_of(p, False, shared) if p in private and p not in targets else p for p in node.parents]
         if first:
             node.parents[:] = parents
@@ -2729,9 +2753,10 @@ def merge_parameter_updates(eg, update_locs):
     return eg
 
 
-def apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape):
+def apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape, updatesrcs=()):
     """The graph rewrites that run after simplification and differentiation, in their fixed order, each under its
-    configuration switch. Returns the new (outputs, update targets)."""
+    configuration switch. `updatesrcs`: the variables that the update targets overwrite. Returns the new (outputs, update
+    targets)."""
     config = core.get_config()
     if config["fuse_conv_dgrad"]:
         outputs_simple, updatetargs_simple = fuse_conv_dgrad(outputs_simple, updatetargs_simple, node2shape)
@@ -2750,7 +2775,7 @@ def apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape):
     if config["fuse_product_sums"]:    # after the batching: the products over all time steps are views by now
         outputs_simple, updatetargs_simple = fuse_product_sums(outputs_simple, updatetargs_simple, node2shape)
     if config["fuse_elementwise"] and config["merge_parameter_updates"]:
-        for (new, old) in split_shared_updates(outputs_simple, updatetargs_simple).items():
+        for (new, old) in split_shared_updates(outputs_simple, updatetargs_simple, updatesrcs).items():
             node2shape[new] = node2shape[old]
     if config["fuse_elementwise"]:
         if config["fuse_rows"] and config["fuse_flat_index_rows"]:
@@ -2774,7 +2799,7 @@ def apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape):
 def rewrite_for_execution(outputs_simple, updatetargs_simple, updatesrcs, node2shape):
     """apply_graph_rewrites, then the rewrites over the finished chains: over time steps, and into the products."""
     config = core.get_config()
-    outputs_simple, updatetargs_simple = apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape)
+    outputs_simple, updatetargs_simple = apply_graph_rewrites(outputs_simple, updatetargs_simple, node2shape, updatesrcs)
     if config["fuse_elementwise"] and config["fuse_rows"] and config["batch_summed_products"]:
         outputs_simple, updatetargs_simple = batch_row_chains(outputs_simple, updatetargs_simple, node2shape)
     # fuse_rows switches everything that adds up in another order than the separate Ops

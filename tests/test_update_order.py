@@ -1,0 +1,61 @@
+"""What a step reads of a variable that it also overwrites: the compiled instruction list, executed on numpy arrays
+(tests/host_run.py), against the oracle, which evaluates everything before it updates anything. Both evaluate an operation
+by the same function, so results are the same bits unless a comment says otherwise."""
+import numpy as np
+import pytest
+
+import cgt_b200 as cgt
+from cgt_b200 import core, nn
+from oracle import cpu_backend
+from tests.host_run import HostRun
+
+
+def _var(rs, *shape):
+    return cgt.shared((rs.randn(*shape) * 0.3).astype("f4"), fixed_shape_mask="all")
+
+
+def _same_as_oracle(inputs, outputs, updates, steps=4, exact=True):
+    run, oracle = HostRun(inputs, outputs, updates), cpu_backend.function(inputs, outputs, updates=updates)
+    for step in range(steps):
+        rs = np.random.RandomState(step)
+        args = [(rs.randn(*x.get_fixed_shape()) * 0.3).astype("f4") for x in inputs]
+        pairs = list(zip(run(*args), oracle(*args))) + [(run.value(v), oracle.get_value(v)) for (v, _new) in updates]
+        for (i, (got, want)) in enumerate(pairs):
+            if exact:
+                assert np.array_equal(got, want), (step, i)
+            else:   # the sums are added up in another order: at most n * eps of the sum of their terms, all positive here
+                np.testing.assert_allclose(got, want, rtol=2000 * np.finfo("f4").eps)
+    return run
+
+
+OPTIMIZERS = {"sgd": dict(learning_rate=0.1), "momentum": dict(learning_rate=0.1), "nesterov_momentum": dict(learning_rate=0.1), "adagrad": {},
+              "rmsprop": {}, "adadelta": {}, "adam": {}}
+
+
+@pytest.mark.parametrize("merge", [True, False])
+@pytest.mark.parametrize("name", sorted(OPTIMIZERS))
+def test_optimizers(name, merge):
+    rs = np.random.RandomState(0)
+    x = cgt.matrix("x", fixed_shape=(32, 24))
+    (W, b, V) = (_var(rs, 24, 40), _var(rs, 1, 40), _var(rs, 40, 10))
+    loss = cgt.square(cgt.tanh(cgt.broadcast("+", x.dot(W), b, "xx,1x")).dot(V)).sum() / 32.0
+    with cgt.scoped_update_config(merge_parameter_updates=merge):
+        _same_as_oracle([x], [loss], getattr(nn, name)(loss, [W, b, V], **OPTIMIZERS[name]))
+
+
+def test_a_shared_operation_on_overwritten_variables_runs_once():
+    rs = np.random.RandomState(0)
+    (a, b, p) = (_var(rs, 33, 5), _var(rs, 33, 5), _var(rs, 33, 5))
+    s = 0.1 * (a + b)
+    _same_as_oracle([], [], [(a, a - s), (b, b - s)])
+    s = 0.1 * (a + cgt.tanh(p * 0.5))   # only tanh(p / 2) may be repeated, and p is not overwritten
+    _same_as_oracle([], [], [(a, a - s), (b, b - s)])
+
+
+def test_a_gradient_that_two_parameters_share_is_one_launch():
+    rs = np.random.RandomState(0)
+    g = cgt.matrix("g", fixed_shape=(33, 5))
+    (a, b) = (_var(rs, 33, 5), _var(rs, 33, 5))
+    step = 0.1 * cgt.tanh(g)
+    run = _same_as_oracle([g], [], [(a, a - step), (b, b - step)])
+    assert [op.k for op in run.ops() if isinstance(op, core.MultiFusedElwise)] == [2]
