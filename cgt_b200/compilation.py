@@ -287,6 +287,48 @@ def variables_read(node):
     return set().union(*[variables_seen(par) for (pos, par) in enumerate(node.parents) if pos not in skip])
 
 
+class UpdateOrder(object):
+    """What has to run before what in a step that overwrites variables: operands before their readers, and every reader of a
+    variable before the update that overwrites it (unless it needs the new value as well, see _update_control_deps).
+
+    A rewrite that makes one instruction of several nodes moves what they read to one place. ``closes_cycle(group)``:
+    something that has to run after one of them has to run before another; they must stay apart. ``join(group)``: they are
+    one from now on."""
+
+    def __init__(self, outputs, updatetargs, updatesrcs):
+        nodes = core.topsorted(list(outputs) + list(updatetargs))
+        number = {t: i for (i, t) in enumerate(updatetargs)}
+        target_of = dict(zip(updatesrcs, updatetargs))
+        self.later = defaultdict(list)
+        needs = {}     # node -> bit set of the update targets that it is or depends on
+        for node in nodes:
+            needs[node] = 1 << number[node] if node in number else 0
+            for par in node.parents:
+                needs[node] |= needs[par]
+                self.later[par].append(node)
+            for v in variables_read(node):
+                t = target_of.get(v)
+                if t is not None and not (needs[node] >> number[t]) & 1:
+                    self.later[node].append(t)
+
+    def closes_cycle(self, group):
+        (group, seen) = (set(group), set())
+        stack = [n for m in group for n in self.later[m] if n not in group]
+        while stack:
+            n = stack.pop()
+            if n in group:
+                return True
+            if n not in seen:
+                seen.add(n)
+                stack.extend(self.later[n])
+        return False
+
+    def join(self, group):
+        for (a, b) in zip(group[:-1], group[1:]):
+            self.later[a].append(b)
+            self.later[b].append(a)
+
+
 def view_leading_slices(outputs, updatetargs, node2shape):
     """GetSli along axis 0 with step 1 and constant bounds -> LeadingSlice: the rows of a C-contiguous array are contiguous,
     so the slice is a view at an offset instead of a copy kernel. Only where the source cannot change under the view:
@@ -699,7 +741,9 @@ def fuse_product_chains(outputs, updatetargs, updatesrcs, node2shape):
     """An elementwise chain (FusedElwise, or a single elementwise node) one of whose inputs is a Mul22 that nothing else
     reads -> Mul22Chain: the chain runs in the output stage of the product, element by element as before, so no bit
     changes; one launch and one trip through memory less. For products of the FMA kernels. An update target may be such a
-    chain (p - lr * dW) unless the product itself reads the variable that is overwritten."""
+    chain (p - lr * dW) unless the product itself reads the variable that is overwritten. The product's operands are read
+    where the chain runs: not where that is too late (a - U.W' for an `a` that needs the new value of U) or would have
+    to be before itself (both updates of a factorisation U.V: each gradient is a product with the other's old value)."""
     all_out = list(outputs) + list(updatetargs)
     nodes = core.topsorted(all_out)
     children = defaultdict(list)
@@ -708,7 +752,8 @@ def fuse_product_chains(outputs, updatetargs, updatesrcs, node2shape):
             children[par].append(node)
     out_set = set(all_out)
     overwrites = dict(zip(updatetargs, updatesrcs))
-    replace, taken = {}, set()
+    order = UpdateOrder(outputs, updatetargs, updatesrcs)
+    replace = {}
     for node in nodes:
         if node.is_input() or node.ndim not in (0, 2) and not is_tuple(node):
             continue
@@ -747,13 +792,14 @@ def fuse_product_chains(outputs, updatetargs, updatesrcs, node2shape):
             variant = product_variant("f4", src.op.tA, src.op.tB, shp[0], shp[1], K) if K >= 1 else -1
             if variant < 0:
                 continue
-            if node in overwrites and overwrites[node] in src.parents:
+            if node in overwrites and overwrites[node] in src.parents or order.closes_cycle([src, node]):
                 continue
             if best is None or K > best[1]:
                 best = (k, K, variant)
         if best is None:
             continue
         product = inputs[best[0]]
+        order.join([product, node])
         others = [p for (k, p) in enumerate(inputs) if k != best[0]]
         new = core.Result(core.Mul22Chain(product.op.tA, product.op.tB, chain, best[0], shp, best[2]), list(product.parents) + others)
         node2shape[new] = node2shape[node]

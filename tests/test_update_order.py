@@ -59,3 +59,23 @@ def test_a_gradient_that_two_parameters_share_is_one_launch():
     step = 0.1 * cgt.tanh(g)
     run = _same_as_oracle([g], [], [(a, a - step), (b, b - step)])
     assert [op.k for op in run.ops() if isinstance(op, core.MultiFusedElwise)] == [2]
+
+
+def test_factorisation():
+    """X ~ U.V by gradient steps: each factor's gradient is a product with the other's old value."""
+    rs = np.random.RandomState(0)
+    X = cgt.matrix("X", fixed_shape=(64, 48))
+    (U, V) = (_var(rs, 64, 32), _var(rs, 32, 48))
+    loss = cgt.square(X - U.dot(V)).sum()
+    run = _same_as_oracle([X], [loss], nn.sgd(loss, [U, V], 0.01))
+    # X - U.V and one of the updates carry their chains; the other's product has to run before the first update
+    assert sum(isinstance(op, core.Mul22Chain) for op in run.ops()) == 2
+
+
+def test_a_product_with_the_old_value_runs_before_the_update():
+    rs = np.random.RandomState(0)
+    A = cgt.matrix("A", fixed_shape=(64, 64))
+    (v, p) = (_var(rs, 64, 64), _var(rs, 64, 64))
+    new = 0.9 * v - 0.1 * cgt.tanh(v)
+    _same_as_oracle([A], [], [(v, new), (p, p - 0.5 * A.dot(v) + new)])
+    _same_as_oracle([A], [v.dot(A) - new], [(v, new)])
