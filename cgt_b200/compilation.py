@@ -792,7 +792,10 @@ def fuse_product_chains(outputs, updatetargs, updatesrcs, node2shape):
             variant = product_variant("f4", src.op.tA, src.op.tB, shp[0], shp[1], K) if K >= 1 else -1
             if variant < 0:
                 continue
-            if node in overwrites and overwrites[node] in src.parents or order.closes_cycle([src, node]):
+            # blocks of one launch would read rows of the variable, or of a view of it, that others are writing
+            if node in overwrites and overwrites[node] in variables_read(src):
+                continue
+            if order.closes_cycle([src, node]):
                 continue
             if best is None or K > best[1]:
                 best = (k, K, variant)

@@ -79,3 +79,13 @@ def test_a_product_with_the_old_value_runs_before_the_update():
     new = 0.9 * v - 0.1 * cgt.tanh(v)
     _same_as_oracle([A], [], [(v, new), (p, p - 0.5 * A.dot(v) + new)])
     _same_as_oracle([A], [v.dot(A) - new], [(v, new)])
+
+
+@pytest.mark.parametrize("view", ["itself", "slice", "reshape"])
+def test_a_chain_does_not_overwrite_what_its_product_multiplies(view):
+    rs = np.random.RandomState(0)
+    W = _var(rs, 64, 64)
+    A = cgt.matrix("A", fixed_shape=(64, 16 if view == "slice" else 64))
+    part = {"itself": W, "slice": W[16:32], "reshape": W.reshape([32, 128]).reshape([64, 64])}[view]
+    _same_as_oracle([A], [], [(W, cgt.tanh(A.dot(part)))])
+    _same_as_oracle([A], [], [(W, W - 0.1 * A.dot(part))])
