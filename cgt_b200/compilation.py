@@ -2737,9 +2737,24 @@ def merge_parameter_updates(eg, update_locs):
     """Instruction-list pass: the update instructions of a step that run one and the same single-output FusedElwise
     program on float32 tensors / scalars (SGD: p - lr * g for every parameter) become ONE MultiFusedElwise instruction
     at the position of the last of them. `update_locs`: indices of the memory locations that updates write (the
-    variables' own storage). An update is moved only if no instruction between its old and its new position touches its
-    result location, so every reader still sees the value it saw before."""
+    variables' own storage). An update is moved only if no instruction between its old and its new position touches the
+    memory of its result, nor writes memory that it reads, itself or through a view: every reader still sees the value it
+    saw before. Two updates of one launch run side by side, so neither may read what the other writes."""
     instrs = eg.instrs
+    holds = {}    # location -> the locations whose memory it may be: its own, or those that it views
+    for ins in instrs:
+        held = holds.setdefault(ins.write_loc.index, {ins.write_loc.index})
+        if isinstance(ins, (ReturnByVal, BuildTup)):
+            held.update(*[holds[r.index] for r in ins.read_locs if r.index in holds])
+
+    def memory(locs):
+        return set().union(*[holds[loc.index] for loc in locs]) if locs else set()
+
+    def written_by(ins):
+        if isinstance(ins, (ReturnByVal, BuildTup, Alloc, LoadArgument)):
+            return set()
+        extra = ins.read_locs[len(ins.read_locs) - ins.op.k + 1:] if isinstance(ins.op, core.MultiFusedElwise) else []
+        return memory([ins.write_loc] + list(extra))
     groups = defaultdict(list)
     for (i, ins) in enumerate(instrs):
         if not isinstance(ins, ReturnByRef) or not isinstance(ins.op, core.FusedElwise) or ins.once:
@@ -2757,19 +2772,9 @@ def merge_parameter_updates(eg, update_locs):
         last = idxs[-1]
         movable = []
         for i in idxs:
-            w = instrs[i].write_loc.index
-            ok = True
-            for j in range(i + 1, last + 1):
-                other = instrs[j]
-                if j in idxs:
-                    if any(r.index == w for r in other.read_locs if j != i) and w != other.write_loc.index:
-                        ok = False
-                    continue
-                locs = [r.index for r in getattr(other, "read_locs", [])] + [other.write_loc.index]
-                if w in locs:
-                    ok = False
-                    break
-            if ok:
+            result, reads = written_by(instrs[i]), memory(instrs[i].read_locs)
+            if all(not (result & memory(list(getattr(instrs[j], "read_locs", [])) + [instrs[j].write_loc])) and
+                   not (reads & written_by(instrs[j])) for j in range(i + 1, last + 1)):
                 movable.append(i)
         movable = movable[:24]
         if len(movable) < 2:

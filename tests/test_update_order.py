@@ -89,3 +89,21 @@ def test_a_chain_does_not_overwrite_what_its_product_multiplies(view):
     part = {"itself": W, "slice": W[16:32], "reshape": W.reshape([32, 128]).reshape([64, 64])}[view]
     _same_as_oracle([A], [], [(W, cgt.tanh(A.dot(part)))])
     _same_as_oracle([A], [], [(W, W - 0.1 * A.dot(part))])
+
+
+def test_merged_updates_do_not_read_each_others_variables():
+    """Every kind of order between updates of one form: p reads v before it changes, d as well, q reads w's new value."""
+    rs = np.random.RandomState(0)
+    g = cgt.matrix("g", fixed_shape=(33, 5))
+    (v, p, d) = (_var(rs, 33, 5), _var(rs, 33, 5), _var(rs, 33, 5))
+    _same_as_oracle([g], [], [(p, p - 0.1 * v), (v, v - 0.1 * g)])
+    _same_as_oracle([g], [], [(v, v - 0.1 * g), (p, p - 0.1 * v)])
+    s = 0.1 * v
+    _same_as_oracle([g], [], [(p, p - s), (d, d - s), (v, v - 0.2 * g)])
+    new = v - 0.1 * g
+    _same_as_oracle([g], [], [(v, new), (p, p - 0.1 * new), (d, d - 0.1 * g)])
+    h = cgt.matrix("h", fixed_shape=(5, 33))
+    (t, u) = (_var(rs, 5, 33), _var(rs, 33, 5))   # through views of each other
+    _same_as_oracle([h], [], [(u, u - 0.1 * t.reshape([33, 5])), (t, t - 0.1 * h)])
+    run = _same_as_oracle([g], [], [(x, x - 0.1 * g) for x in (v, p, d)])
+    assert [op.k for op in run.ops() if isinstance(op, core.MultiFusedElwise)] == [3]
