@@ -930,9 +930,9 @@ def batch_row_chains(outputs, updatetargs, node2shape):
     return _rewire(outputs, updatetargs, replace)
 
 
-def fuse_square_sums(outputs, updatetargs, node2shape):
+def fuse_square_sums(outputs, updatetargs, updatesrcs, node2shape):
     """Sum(square(x)) over all axes of several float32 arrays, none of which needs another's sum -> SumSquares, one launch
-    for all of them. Arrays of up to 2^20 elements: a larger one keeps more blocks busy than the eight it has here."""
+    for all of them, unless it would come too late for one of them (the norms of a variable's old and new value). Arrays of up to 2^20 elements: a larger one keeps more blocks busy than the eight it has here."""
     all_out = list(outputs) + list(updatetargs)
     nodes = core.topsorted(all_out)
     children = defaultdict(list)
@@ -940,7 +940,8 @@ def fuse_square_sums(outputs, updatetargs, node2shape):
         for par in node.parents:
             children[par].append(node)
     out_set = set(all_out)
-    found, reached = [], set()
+    order = UpdateOrder(outputs, updatetargs, updatesrcs)
+    found, group, reached = [], [], set()
     for node in nodes:
         if any(p in reached for p in node.parents):
             reached.add(node)
@@ -952,7 +953,10 @@ def fuse_square_sums(outputs, updatetargs, node2shape):
         (x, shp) = (sq.parents[0], _static_shape(node2shape[sq]))
         if x.dtype != "f4" or shp is None or len(node.op.axes) != len(shp) or not 1 <= np.prod(shp, dtype=np.int64) <= 1 << 20 or x in reached:
             continue
+        if order.closes_cycle(group + [node, sq]):
+            continue
         found.append((node, x))
+        group += [node, sq]
         reached.add(node)
     if len(found) < 2:
         return list(outputs), list(updatetargs)
@@ -2858,7 +2862,7 @@ def rewrite_for_execution(outputs_simple, updatetargs_simple, updatesrcs, node2s
         outputs_simple, updatetargs_simple = batch_row_chains(outputs_simple, updatetargs_simple, node2shape)
     # fuse_rows switches everything that adds up in another order than the separate Ops
     if config["fuse_square_sums"] and config["fuse_rows"]:
-        outputs_simple, updatetargs_simple = fuse_square_sums(outputs_simple, updatetargs_simple, node2shape)
+        outputs_simple, updatetargs_simple = fuse_square_sums(outputs_simple, updatetargs_simple, updatesrcs, node2shape)
     if config["fuse_elementwise"] and config["fuse_rows"] and config["fuse_recurrences"] and config["jit_fused_elementwise"]:
         outputs_simple, updatetargs_simple = fuse_recurrences(outputs_simple, updatetargs_simple, node2shape)
     # fuse_product_sums switches every use of the products' output stage

@@ -107,3 +107,12 @@ def test_merged_updates_do_not_read_each_others_variables():
     _same_as_oracle([h], [], [(u, u - 0.1 * t.reshape([33, 5])), (t, t - 0.1 * h)])
     run = _same_as_oracle([g], [], [(x, x - 0.1 * g) for x in (v, p, d)])
     assert [op.k for op in run.ops() if isinstance(op, core.MultiFusedElwise)] == [3]
+
+
+def test_norms_of_an_old_and_a_new_value():
+    rs = np.random.RandomState(0)
+    B = cgt.matrix("B", fixed_shape=(33, 5))
+    (U, V, W) = (_var(rs, 33, 5), _var(rs, 40, 7), _var(rs, 1, 9))
+    new = U - 0.1 * cgt.tanh(U - B)
+    run = _same_as_oracle([B], [cgt.square(x).sum() * 1.0 for x in (U, V, new, W)], [(U, new), (V, V * 0.9)], exact=False)
+    assert [len(op.ndims) for op in run.ops() if isinstance(op, core.SumSquares)] == [3]   # all but the new value's
