@@ -2501,7 +2501,7 @@ def _update_control_deps(outputs_all, updates):
             children[p].append(node)
     extra = {}
     for (before, after) in updates:
-        # descendants of `after` cannot be ordered before it
+        # descendants of `after` cannot be ordered before it (keep_old_values gives them a copy of the old value)
         desc = set([after])
         for node in nodelist:
             if any(p in desc for p in node.parents):
@@ -2520,6 +2520,70 @@ def _update_control_deps(outputs_all, updates):
                 stack.extend(children[c])
         extra[after] = readers
     return extra
+
+
+def _in_place_unsafe(node):
+    """Positions of the operands whose memory the operation may still read at one place when it has written another: all of
+    them, but for elementwise operations those that are views of a part."""
+    op = node.op
+    if op.writes_to_input >= 0:
+        return [pos for pos in range(len(node.parents)) if pos != op.writes_to_input]
+    product = 2 if isinstance(op, core.Mul22Chain) else 0
+    if not product and not isinstance(op, (core.ElwiseUnary, core.ElwiseBinary, core.FusedElwise)):
+        return list(range(len(node.parents)))
+
+    def whole(par):
+        while not par.is_input() and isinstance(par.op, core.Reshape):
+            par = par.parents[0]
+        return par.is_input() or par.op.return_type == "byref"
+    return [pos for (pos, par) in enumerate(node.parents) if pos < product or not whole(par)]
+
+
+def keep_old_values(outputs_all, updates, node2dev, node2shape):
+    """Every operation sees the variables as they were before the call: an operation that reads a variable and cannot run
+    before the variable's update, because it needs the new value too or because two updates need each other's variable,
+    reads a copy taken at the beginning; so does an update that would read its own variable in places that it has
+    written already. The fusions avoid making such operations; this is what holds whatever they do."""
+    nodes = core.topsorted(outputs_all)
+    later, readers = defaultdict(list), defaultdict(list)
+    for node in nodes:
+        for par in node.parents:
+            later[par].append(node)
+        for v in variables_read(node):
+            readers[v].append(node)
+    for (v, target) in updates:
+        copies = {}
+
+        def old(node):
+            """`node`, which sees v, over v's copy"""
+            if node is not v and (node.is_input() or v not in variables_seen(node)):
+                return node
+            if node not in copies:
+                if node is v:
+                    name = "cast_to_" + v.dtype
+                    new = core.Result(core.ElwiseUnary(name, core.UnaryInfo(name, None, False, v.dtype, None, "x")), [v])
+                else:
+                    new = core.Result(node.op, [old(par) for par in node.parents], typ=node.typ)
+                new.props.update(node.props)
+                (node2dev[new], node2shape[new]) = (node2dev[node], node2shape[node])
+                copies[node] = new
+            return copies[node]
+        (reached, stack) = ({target}, [target])
+        while stack:
+            for n in later[stack.pop()]:
+                if n not in reached:
+                    reached.add(n)
+                    stack.append(n)
+        for node in readers[v]:
+            if node is target:
+                late = _in_place_unsafe(node)
+            elif node in reached:
+                late = range(len(node.parents))
+            else:
+                later[node].append(target)
+                continue
+            for pos in late:
+                node.parents[pos] = old(node.parents[pos])
 
 
 def _transport_schedule(outputs_all, updatetargs, node2dev):
@@ -2884,6 +2948,7 @@ def execution_graph(inputs, outputs, updates, givens):
     add_transports(nodelist, node2dev, node2shape)
 
     updates_simple = list(zip(updatesrcs, updatetargs_simple))
+    keep_old_values(all_out, updates_simple, node2dev, node2shape)
     extra = _update_control_deps(all_out, updates_simple)
     first, last = _transport_schedule(all_out, updatetargs_simple, node2dev)
     for node in last:

@@ -28,6 +28,10 @@ def _same_as_oracle(inputs, outputs, updates, steps=4, exact=True):
     return run
 
 
+def _copies(run):
+    return sum(isinstance(op, core.ElwiseUnary) and op.opname == "cast_to_f4" for op in run.ops())
+
+
 OPTIMIZERS = {"sgd": dict(learning_rate=0.1), "momentum": dict(learning_rate=0.1), "nesterov_momentum": dict(learning_rate=0.1), "adagrad": {},
               "rmsprop": {}, "adadelta": {}, "adam": {}}
 
@@ -40,7 +44,8 @@ def test_optimizers(name, merge):
     (W, b, V) = (_var(rs, 24, 40), _var(rs, 1, 40), _var(rs, 40, 10))
     loss = cgt.square(cgt.tanh(cgt.broadcast("+", x.dot(W), b, "xx,1x")).dot(V)).sum() / 32.0
     with cgt.scoped_update_config(merge_parameter_updates=merge):
-        _same_as_oracle([x], [loss], getattr(nn, name)(loss, [W, b, V], **OPTIMIZERS[name]))
+        run = _same_as_oracle([x], [loss], getattr(nn, name)(loss, [W, b, V], **OPTIMIZERS[name]))
+    assert not _copies(run)
 
 
 def test_a_shared_operation_on_overwritten_variables_runs_once():
@@ -68,6 +73,7 @@ def test_factorisation():
     (U, V) = (_var(rs, 64, 32), _var(rs, 32, 48))
     loss = cgt.square(X - U.dot(V)).sum()
     run = _same_as_oracle([X], [loss], nn.sgd(loss, [U, V], 0.01))
+    assert not _copies(run)
     # X - U.V and one of the updates carry their chains; the other's product has to run before the first update
     assert sum(isinstance(op, core.Mul22Chain) for op in run.ops()) == 2
 
@@ -116,3 +122,39 @@ def test_norms_of_an_old_and_a_new_value():
     new = U - 0.1 * cgt.tanh(U - B)
     run = _same_as_oracle([B], [cgt.square(x).sum() * 1.0 for x in (U, V, new, W)], [(U, new), (V, V * 0.9)], exact=False)
     assert [len(op.ndims) for op in run.ops() if isinstance(op, core.SumSquares)] == [3]   # all but the new value's
+
+
+@pytest.mark.parametrize("fuse", [True, False])
+def test_what_needs_old_and_new_value(fuse):
+    """v and its new value meet in one operation, or in one chain after fusion; updates that need each other's variable."""
+    rs = np.random.RandomState(0)
+    (v, p, n) = (_var(rs, 33, 5), _var(rs, 33, 5), _var(rs, 12, 5))
+    new = 0.9 * v - 0.1 * cgt.tanh(v)
+    with cgt.scoped_update_config(fuse_elementwise=fuse):
+        _same_as_oracle([], [cgt.square(v * new)], [(v, new), (p, p - v * new)])
+        _same_as_oracle([], [], [(v, new), (p, p - 0.5 * v + new)])
+        _same_as_oracle([], [cgt.concatenate([v[0:9], new], axis=0) * 2.0], [(v, new)])
+        _same_as_oracle([], [], [(v, v - p), (p, p - v)])
+        _same_as_oracle([], [], [(v, v - p), (p, p + cgt.concatenate([n, v[3:24]], axis=0)), (n, n * v[0:12])])
+
+
+def test_updates_that_read_their_variable_elsewhere():
+    rs = np.random.RandomState(0)
+    x = cgt.matrix("x", fixed_shape=(1, 40))
+    A = cgt.matrix("A", fixed_shape=(40, 40))
+    (W, last) = (_var(rs, 8, 40), _var(rs, 40, 40))
+    _same_as_oracle([x], [], [(W, cgt.concatenate([x, W[0:7]], axis=0))])          # the last eight rows
+    _same_as_oracle([A], [], [(last, last.dot(A)), (W, W.dot(A))])
+    _same_as_oracle([A], [], [(last, last.T)])
+    _same_as_oracle([x], [], [(W, W - cgt.repeat(W[0:1], 8, axis=0))])
+    _same_as_oracle([], [], [(W, nn.softmax(W))], exact=False)
+
+
+def test_ordinary_steps_take_no_copies():
+    """The copies are for steps that have no other order: none of the configurations and optimizers has them."""
+    from cgt_b200 import compilation, configs
+    small = {"mlp": dict(batch=8), "cifar": dict(batch=2), "wide": dict(batch=2), "lstm": dict(seq_len=4, batch=4), "vae": dict(batch=5)}
+    for (name, kw) in small.items():
+        cfg = configs.BUILDERS[name](**kw)
+        eg = compilation.execution_graph(cfg.inputs, [cfg.loss] + list(cfg.extra_outputs), cfg.updates, [])[0]
+        assert not any(isinstance(getattr(i, "op", None), core.ElwiseUnary) and i.op.opname == "cast_to_f4" for i in eg.instrs), name
