@@ -333,13 +333,16 @@ def view_leading_slices(outputs, updatetargs, node2shape):
     """GetSli along axis 0 with step 1 and constant bounds -> LeadingSlice: the rows of a C-contiguous array are contiguous,
     so the slice is a view at an offset instead of a copy kernel. Only where the source cannot change under the view:
     it is an argument's device copy or any other node that no instruction writes into (no update target, no IncSli /
-    IncFlatIndices base)."""
+    IncFlatIndices base), or a shared variable whose slice is read within the step (before the variable's update): not one
+    that the caller gets, who looks at it after the update."""
     all_out = list(outputs) + list(updatetargs)
     nodes = core.topsorted(all_out)
-    written = set()
-    for node in nodes:
+    written, handed_out = set(), set(all_out)
+    for node in reversed(nodes):
         if not node.is_input() and node.op.writes_to_input >= 0:
             written.add(node.parents[node.op.writes_to_input])
+        if node in handed_out and not node.is_input() and node.op.return_type == "byval":
+            handed_out.update(node.parents)
     replace = {}
     for node in nodes:
         if node.is_input() or not isinstance(node.op, core.GetSli) or node.op.axis != 0 or node in all_out:
@@ -351,8 +354,8 @@ def view_leading_slices(outputs, updatetargs, node2shape):
         (a, b, st) = (int(start.op.value), int(stop.op.value), int(step.op.value))
         if st != 1 or xshp is None or not (0 <= a <= b <= xshp[0]) or x in written or x in updatetargs:
             continue
-        if not x.is_input() and isinstance(x.op, core.InMemoryData):
-            continue   # a shared variable can be updated in place while the view is alive
+        if x.is_data() and node in handed_out:
+            continue
         new = core.Result(core.LeadingSlice(), [x, start, stop])
         node2shape[new] = node2shape[node]
         new.props.update(node.props)

@@ -158,3 +158,12 @@ def test_ordinary_steps_take_no_copies():
         cfg = configs.BUILDERS[name](**kw)
         eg = compilation.execution_graph(cfg.inputs, [cfg.loss] + list(cfg.extra_outputs), cfg.updates, [])[0]
         assert not any(isinstance(getattr(i, "op", None), core.ElwiseUnary) and i.op.opname == "cast_to_f4" for i in eg.instrs), name
+
+
+def test_a_slice_that_is_handed_out_keeps_its_old_value():
+    rs = np.random.RandomState(0)
+    W = _var(rs, 8, 40)
+    run = _same_as_oracle([], [W[2:5], W[0:3].reshape([12, 10])], [(W, W * 0.9)])
+    assert not any(isinstance(op, core.LeadingSlice) for op in run.ops())
+    run = _same_as_oracle([], [cgt.tanh(W[2:5])], [(W, W * 0.9)])
+    assert any(isinstance(op, core.LeadingSlice) for op in run.ops())
