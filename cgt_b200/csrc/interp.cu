@@ -116,6 +116,7 @@ struct cgtbInterp {
   long out_stage_cap = 0;
   std::vector<void*> out_host;          // per result: its bytes in host memory, or null (not an array on the device)
   std::vector<long> out_offset;
+  std::vector<char> out_is_argument;    // per result: it is, or views, one of the call's arguments
   std::vector<cgtArray*> out_array;     // the array that was copied to out_host
   long last_host_ns = 0;                // host time of the last run up to the final wait for the stream
   long steady_runs = 0;
@@ -334,6 +335,7 @@ CGTB_API cgtbInterp* cgtb_interp_new(cgtbGraph* g, int n_out, const long* out_lo
       if (dep) from_arg[(size_t)in.write.idx] |= dep;
     }
     it->args_read_in_place = in_place;
+    for (auto& o : it->outs) it->out_is_argument.push_back(from_arg[(size_t)o.idx] != 0);
   }
   build_spans(it);
   return it;
@@ -466,9 +468,10 @@ static uint64_t span_key(cgtbInterp* it, const Span& s) {
   }
   if (s.collects) {
     h = mix(h, (uint64_t)(uintptr_t)it->out_stage);
-    for (auto& o : it->outs) {
-      cgtObject* obj = get(it, o);
-      if (obj && obj->kind() == cgtObject::ArrayKind && ((cgtArray*)obj)->devtype() == cgtGPU) h = key_of_object(h, obj, cgtbGPU);
+    for (size_t i = 0; i < it->outs.size(); ++i) {
+      cgtObject* obj = get(it, it->outs[i]);
+      if (obj && obj->kind() == cgtObject::ArrayKind && ((cgtArray*)obj)->devtype() == cgtGPU && !it->out_is_argument[i])
+        h = key_of_object(h, obj, cgtbGPU);
     }
   }
   return h;
@@ -679,14 +682,16 @@ static void add_copy_out(CopyJobs& jobs, const void* src, void* dst, long nbytes
   }
   jobs.job[jobs.n++] = CopyJob{src, dst, nbytes};
 }
-// Place of every device result in the pinned result block (grown here, outside captures).
+// Place of every device result in the pinned result block (grown here, outside captures). An argument that the function
+// hands back is not copied by the graph, which would keep the address that it had when the graph was captured: the
+// caller reads it from the object that this call got.
 static int place_outputs(cgtbInterp* it) {
   long total = 0;
   it->out_offset.assign(it->outs.size(), -1);
   it->out_array.assign(it->outs.size(), nullptr);
   for (size_t i = 0; i < it->outs.size(); ++i) {
     cgtObject* o = get(it, it->outs[i]);
-    if (!o || o->kind() != cgtObject::ArrayKind || ((cgtArray*)o)->devtype() != cgtGPU) continue;
+    if (!o || o->kind() != cgtObject::ArrayKind || ((cgtArray*)o)->devtype() != cgtGPU || it->out_is_argument[i]) continue;
     it->out_offset[i] = total;
     it->out_array[i] = (cgtArray*)o;
     total += (((cgtArray*)o)->nbytes() + 63) & ~63L;

@@ -43,3 +43,19 @@ def test_more_arguments_and_results_than_one_copy_kernel_takes(rt):
         vals = [rs.randn(3 + i).astype("f4") for i in range(40)]
         for (v, got) in zip(vals, f(*vals)):
             assert np.array_equal(got, v + np.float32(1))
+
+
+@pytest.mark.parametrize("n", [6, 300 * KB])
+def test_an_argument_that_is_handed_back(rt, n):
+    """The result is the array of this call: also when another array of the same shape was there when the step's graph was
+    captured, and when the result is a view of the argument."""
+    x = cgt.vector("x", fixed_shape=(n,))
+    f = cgt.function([x], [x, x * 2.0, x.reshape([2, n // 2])])
+    rs = np.random.RandomState(0)
+    vals = [rs.randn(n).astype("f4") for _ in range(3)]
+    on_device = [runtime.device_array(v) for v in vals]
+    for i in [0, 0, 0, 0, 0, 1, 1, 2, 0, 1, 2, 2]:
+        (same, twice, view) = f(on_device[i])
+        assert np.array_equal(twice, vals[i] * 2) and np.array_equal(same, vals[i]) and np.array_equal(view, vals[i].reshape(2, -1)), i
+    for i in [0, 1, 2, 0]:
+        assert np.array_equal(f(vals[i])[0], vals[i])
