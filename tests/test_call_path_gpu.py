@@ -59,3 +59,19 @@ def test_an_argument_that_is_handed_back(rt, n):
         assert np.array_equal(twice, vals[i] * 2) and np.array_equal(same, vals[i]) and np.array_equal(view, vals[i].reshape(2, -1)), i
     for i in [0, 1, 2, 0]:
         assert np.array_equal(f(vals[i])[0], vals[i])
+
+
+@pytest.mark.parametrize("sizes", [(2, 2), (2, 3, 1), (40,), (70, 2)])
+def test_large_host_arrays_in_one_call(rt, sizes):
+    """Arrays above a megabyte share the pinned staging memory, above 32 MB in several stretches: the second one finds the
+    first one's copies still under way. Doubling is exact."""
+    MB = 1 << 18  # floats
+    xs = [cgt.vector("x%d" % i) for i in range(len(sizes))]
+    f = cgt.function(xs, [cgt.sum(x * 2.0) if i else x * 2.0 for (i, x) in enumerate(xs)])
+    rs = np.random.RandomState(1)
+    for run in range(4):
+        vals = [rs.randint(-8, 8, size=n * MB + 5).astype("f4") for n in sizes]
+        got = f(*vals)
+        assert np.array_equal(got[0], vals[0] * 2), run
+        for (v, g) in zip(vals[1:], got[1:]):   # whole numbers, every partial sum below 2^24: exact in any order
+            assert g == 2 * v.astype("f8").sum(), run
