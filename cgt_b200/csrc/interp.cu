@@ -59,6 +59,7 @@ struct Instr {
   Klass klass = kMeta;
   bool fired = false;
   bool arg_view = false;  // host bookkeeping on (a view of) an argument: fired in steady runs too
+  bool from_argument = false;  // kUpload: the source is (a view of) an argument, which nothing in the call writes
   ScratchOwner scratch;
   void* stage = nullptr;  // kUpload: pinned copy of the host operand, read by the span's copy kernel
   long stage_cap = 0;
@@ -328,6 +329,7 @@ CGTB_API cgtbInterp* cgtb_interp_new(cgtbGraph* g, int n_out, const long* out_lo
         in_place |= from_arg[(size_t)in.write.idx];
         continue;
       }
+      if (in.klass == kUpload) in.from_argument = from_arg[(size_t)in.reads[0].idx] != 0;
       if (in.klass != kMeta) continue;
       uint64_t dep = in.kind == kLoadArgument ? (1ull << (in.arg_index < 63 ? in.arg_index : 63)) : 0;
       for (auto& r : in.reads) dep |= from_arg[(size_t)r.idx];
@@ -637,7 +639,9 @@ static int fire_span_multistream(cgtbInterp* it, Span& s, cudaStream_t origin) {
 // Copies between host and device: uploads at a span's start, downloads and results at its end
 // ------------------------------------------------------------------------------------------------
 // Host part of an upload (pass 1, in program order): what the copy kernel will read is put in place, or a large host
-// array is sent through the copy engine at once.
+// array is sent through the copy engine at once. The kernel runs after all host instructions of the span, so it may read
+// only what none of them can write: an argument, or a copy made here. A variable's host memory (a learning rate that the
+// call also decays) is copied now, one on the device by a copy that is queued now, ahead of what pass 1 queues after it.
 static int stage_upload(cgtbInterp* it, Span& s, Instr& in) {
   cgtObject *src_o = get(it, in.reads[0]), *dst_o = get(it, in.write);
   if (!src_o || !dst_o) return fail("%s: operand was never produced", in.repr.c_str());
@@ -648,13 +652,9 @@ static int stage_upload(cgtbInterp* it, Span& s, Instr& in) {
   if (nbytes == 0) return 0;
   const void* from = src->data();
   if (src->devtype() == cgtCPU) {
-    const bool pinned = host_block_is_pinned(from);
-    if (nbytes > kKernelCopyBytes) {
-      if (!pinned) return upload_pageable(dst->data(), from, (size_t)nbytes);
-      CGTB_CUDA_TRY(cudaMemcpyAsync(dst->data(), from, (size_t)nbytes, cudaMemcpyHostToDevice, rt().stream));
-      return 0;
-    }
-    if (!pinned) {
+    const bool pinned = host_block_is_pinned(from), large = nbytes > kKernelCopyBytes;
+    if (large && !pinned) return upload_pageable(dst->data(), from, (size_t)nbytes);
+    if (!pinned || !in.from_argument) {
       if (in.stage_cap < nbytes) {
         if (in.stage) cgtb_free(cgtbCPU, in.stage);
         in.stage = cgtb_alloc(cgtbCPU, nbytes);
@@ -664,6 +664,13 @@ static int stage_upload(cgtbInterp* it, Span& s, Instr& in) {
       stage_for_kernel(in.stage, from, (size_t)nbytes);
       from = in.stage;
     }
+    if (large) {
+      CGTB_CUDA_TRY(cudaMemcpyAsync(dst->data(), from, (size_t)nbytes, cudaMemcpyHostToDevice, rt().stream));
+      return 0;
+    }
+  } else if (!in.from_argument) {
+    CGTB_CUDA_TRY(cudaMemcpyAsync(dst->data(), from, (size_t)nbytes, cudaMemcpyDeviceToDevice, rt().stream));
+    return 0;
   }
   s.uploads.job[s.uploads.n++] = CopyJob{from, dst->data(), nbytes};
   return 0;
