@@ -113,6 +113,8 @@ struct cgtbInterp {
   bool prev_run_ok = false;
   uint64_t args_read_in_place = ~0ull;  // arguments whose device buffer a captured instruction reads directly
   std::vector<char> downloaded;         // locations that a device->host copy writes
+  std::vector<long> memory_of;          // per location: the location whose memory it is or views
+  bool by_value_state = false;          // a host value that an instruction takes is overwritten later in the call
   char* out_stage = nullptr;            // pinned block that holds the device results of the last run
   long out_stage_cap = 0;
   std::vector<void*> out_host;          // per result: its bytes in host memory, or null (not an array on the device)
@@ -256,6 +258,7 @@ static void build_spans(cgtbInterp* it) {
     } else {
       int j = i, n_uploads = 0, n_downloads = 0;
       std::vector<char> fresh((size_t)it->g->n_locs, 0);  // copied to the host by this span
+      std::vector<char> taken((size_t)it->g->n_locs, 0);  // host memory that a device instruction reads when it is issued
       while (j < n && !is_barrier(j)) {
         Instr& in = instrs[(size_t)j];
         if (n_downloads) {
@@ -265,6 +268,12 @@ static void build_spans(cgtbInterp* it) {
           if (cut || (in.klass == kDownload && n_downloads == kMaxCopyJobs)) break;
         }
         if (in.klass == kUpload && n_uploads == kMaxCopyJobs) break;
+        // device instructions are issued after the span's host instructions: one that overwrites what they take by
+        // value (the start of a slice that the call moves on) has to wait for the next span
+        if (in.klass == kHostData && taken[(size_t)it->memory_of[(size_t)in.write.idx]]) break;
+        if (in.klass == kDevice)
+          for (auto& r : in.reads)
+            if (r.dev == cgtbCPU) taken[(size_t)it->memory_of[(size_t)r.idx]] = 1;
         if (in.klass == kDownload) {
           ++n_downloads;
           fresh[(size_t)in.write.idx] = 1;
@@ -337,6 +346,16 @@ CGTB_API cgtbInterp* cgtb_interp_new(cgtbGraph* g, int n_out, const long* out_lo
       if (dep) from_arg[(size_t)in.write.idx] |= dep;
     }
     it->args_read_in_place = in_place;
+    it->memory_of.resize((size_t)g->n_locs);
+    for (long l = 0; l < g->n_locs; ++l) it->memory_of[(size_t)l] = l;
+    std::vector<char> taken((size_t)g->n_locs, 0);
+    for (auto& in : g->instrs) {
+      if (in.kind == kReturnByVal && in.klass == kMeta && !in.reads.empty()) it->memory_of[(size_t)in.write.idx] = it->memory_of[(size_t)in.reads[0].idx];
+      if (in.klass == kHostData) it->by_value_state = it->by_value_state || taken[(size_t)it->memory_of[(size_t)in.write.idx]];
+      if (in.klass == kDevice || in.kind == kAlloc)
+        for (auto& r : in.reads)
+          if (r.dev == cgtbCPU) taken[(size_t)it->memory_of[(size_t)r.idx]] = 1;
+    }
     for (auto& o : it->outs) it->out_is_argument.push_back(from_arg[(size_t)o.idx] != 0);
   }
   build_spans(it);
@@ -975,7 +994,8 @@ CGTB_API int cgtb_interp_run(cgtbInterp* it, cgtbObject* args_obj, cgtbObject** 
     }
     const long ver = g_state_version.load(std::memory_order_relaxed);
     static const bool allow = []() { const char* e = getenv("CGTB_STEADY_RUNS"); return !(e && e[0] == '0'); }();
-    it->steady = allow && it->prev_run_ok && !it->prev_run_allocated && it->runs >= 2 && ver == it->state_version_seen &&
+    // a steady run takes host values from the run before: not where the call itself leaves another value for the next one
+    it->steady = allow && !it->by_value_state && it->prev_run_ok && !it->prev_run_allocated && it->runs >= 2 && ver == it->state_version_seen &&
                  sig == it->arg_sig && !(it->flags & CGTB_INTERP_PROFILE);
     it->arg_sig.swap(sig);
     it->state_version_seen = ver;

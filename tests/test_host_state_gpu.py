@@ -38,3 +38,15 @@ def test_a_large_host_variable(rt):
         v = np.random.RandomState(step).randn(n).astype("f4")
         table.op.set_value(v)
         assert np.array_equal(f()[0], v * 2), step
+
+
+@pytest.mark.parametrize("rows,move", [(1, 1), (3, 2)])
+def test_a_cursor_that_moves(rt, rows, move):
+    """x[k:k+rows] with k a host variable that the call moves on: the slice is taken where k was before the call."""
+    k = cgt.shared(np.array(0, "i8"), device=core.Device("cpu", 0))
+    x = cgt.matrix("x", fixed_shape=(40, 5))
+    f = cgt.function([x], [x[k:k + rows] * 2.0], updates=[(k, k + move)])
+    a = np.arange(200, dtype="f4").reshape(40, 5)
+    v = runtime.device_array(a)
+    for step in range(12):
+        assert np.array_equal(f(v)[0], 2 * a[step * move:step * move + rows]), step
