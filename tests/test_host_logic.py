@@ -608,3 +608,53 @@ def test_recurrence_plans_cover_their_extents():
                     assert p["C"] * p["UH"] >= H > (p["C"] - 1) * p["UH"] and p["NC"] == p["UH"] * (N // H)
                     assert p["KG"] * p["KT"] >= KA > (p["KG"] - 1) * p["KT"] and p["KT"] % 4 == 0 and p["KG"] * p["NC"] <= 256
                     assert p["RB"] * p["UH"] <= 256 and 4 * (2 * p["RB"] * p["KG"] * p["KT"] + p["KG"] * p["RB"] * p["NC"]) <= 48 * 1024
+
+
+# ------------------------------------------------------------------------------------------------
+# copies on the host by several threads
+# ------------------------------------------------------------------------------------------------
+def _host_copies(sizes, rounds):
+    lib = runtime.lib()
+    for r in range(rounds):
+        for n in sizes:
+            src = np.random.RandomState(n + r).randint(0, 255, size=n).astype("u1")
+            dst = np.zeros(n, "u1")
+            lib.cgtb_host_copy(ctypes.c_void_p(dst.ctypes.data), ctypes.c_void_p(src.ctypes.data), n)
+            if not np.array_equal(src, dst):
+                return "copy of %d bytes differs" % n
+
+
+def test_host_copies_of_several_callers():
+    """Whoever finds the helper threads busy copies alone; nobody's copy changes how another one is done."""
+    import concurrent.futures
+    sizes = [1, (1 << 20) - 1, 1 << 20, (1 << 20) + 1, (5 << 18) + 77, 9 << 20]
+    with concurrent.futures.ThreadPoolExecutor(4) as pool:
+        assert list(pool.map(lambda k: _host_copies(sizes[k % 2:] + sizes[:k], 8), range(4))) == [None] * 4
+
+
+_COPY_RACE = """
+#include "%s/copy_threads.h"
+static cgtb::CopyThreads g;
+int main() {
+  auto callers = [](bool to_gpu) {
+    std::vector<char> a(4 << 20, 1), b(4 << 20);
+    for (int i = 0; i < 10; ++i) g.copy(b.data(), a.data(), a.size(), to_gpu, [](size_t, size_t) {});
+  };
+  std::thread one(callers, true), two(callers, false);
+  one.join();
+  two.join();
+}
+"""
+
+
+def test_copy_threads_under_the_thread_sanitizer(tmp_path):
+    import subprocess
+    (src, exe) = (tmp_path / "race.cpp", tmp_path / "race")
+    src.write_text(_COPY_RACE % osp.join(ROOT, "cgt_b200", "csrc"))
+    probe = subprocess.run(["c++", "-std=c++17", "-fsanitize=thread", "-x", "c++", "-", "-o", str(tmp_path / "probe")],
+                           input="int main() {}", text=True, capture_output=True)
+    if probe.returncode or subprocess.run(["setarch", "-R", str(tmp_path / "probe")], capture_output=True).returncode:
+        pytest.skip("no thread sanitizer")
+    subprocess.run(["c++", "-std=c++17", "-g", "-O1", "-fsanitize=thread", str(src), "-o", str(exe)], check=True)
+    run = subprocess.run(["setarch", "-R", str(exe)], capture_output=True, text=True, timeout=120)
+    assert run.returncode == 0 and "data race" not in run.stderr, run.stderr[:2000]
