@@ -6,6 +6,7 @@
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -58,7 +59,7 @@ class CopyThreads {
   void copy(char* dst, const char* src, size_t n, bool to_gpu, F in_order) {
     std::unique_lock<std::mutex> owner(owner_, std::try_to_lock);
     const size_t chunks = (n + kChunk - 1) / kChunk;
-    if (!owner.owns_lock() || chunks < 4) {
+    if (!owner.owns_lock() || chunks < 4 || !prepare(chunks)) {
       for (size_t c = 0; c < chunks; ++c) {
         const size_t at = c * kChunk, end = std::min(n, at + kChunk);
         memcpy(dst + at, src + at, end - at);  // alone: a thread's streaming stores are slower than its memcpy
@@ -66,9 +67,6 @@ class CopyThreads {
       }
       return;
     }
-    if (threads_.empty())
-      for (int i = 0; i < kHelpers; ++i) threads_.emplace_back([this] { work(); });
-    if (done_.size() < chunks) done_ = std::vector<std::atomic<char>>(chunks);
     for (size_t c = 0; c < chunks; ++c) done_[c].store(0, std::memory_order_relaxed);
     to_gpu_ = to_gpu;   // the job's fields are the owner's to write, and only while no helper is at work
     dst_ = dst;
@@ -98,6 +96,17 @@ class CopyThreads {
   }
 
  private:
+  // The helpers and a flag per chunk. A process at its limit of threads or memory gets none: false, and the caller copies
+  // alone (an exception must not leave through the C interface). It is tried again by the next copy.
+  bool prepare(size_t chunks) {
+    try {
+      if (done_.size() < chunks) done_ = std::vector<std::atomic<char>>(chunks);
+      threads_.reserve(kHelpers);
+      while (threads_.size() < kHelpers) threads_.emplace_back([this] { work(); });
+    } catch (const std::exception&) {
+    }
+    return done_.size() >= chunks && !threads_.empty();
+  }
   bool one_chunk() {
     const size_t c = next_.fetch_add(1, std::memory_order_relaxed);
     if (c >= chunks_) return false;

@@ -658,3 +658,31 @@ def test_copy_threads_under_the_thread_sanitizer(tmp_path):
     subprocess.run(["c++", "-std=c++17", "-g", "-O1", "-fsanitize=thread", str(src), "-o", str(exe)], check=True)
     run = subprocess.run(["setarch", "-R", str(exe)], capture_output=True, text=True, timeout=120)
     assert run.returncode == 0 and "data race" not in run.stderr, run.stderr[:2000]
+
+
+_COPY_LIMIT = """
+#include "%s/copy_threads.h"
+#include <cstdio>
+#include <sys/resource.h>
+static cgtb::CopyThreads g;
+int main() {
+  std::vector<char> a(4 << 20, 1), b(4 << 20);
+  long pages = 0;
+  FILE* f = fopen("/proc/self/statm", "r");
+  if (!f || fscanf(f, "%%ld", &pages) != 1) return 2;
+  fclose(f);
+  const rlimit now = {(rlim_t)(pages * 4096 + (1 << 20)), (rlim_t)RLIM_INFINITY};  // no room for a thread's stack
+  if (setrlimit(RLIMIT_AS, &now)) return 3;
+  size_t upto = 0;
+  g.copy(b.data(), a.data(), a.size(), false, [&](size_t, size_t end) { upto = end; });
+  return upto == a.size() && a == b ? 0 : 1;
+}
+"""
+
+
+def test_copies_without_helper_threads(tmp_path):
+    import subprocess
+    (src, exe) = (tmp_path / "limit.cpp", tmp_path / "limit")
+    src.write_text(_COPY_LIMIT % osp.join(ROOT, "cgt_b200", "csrc"))
+    subprocess.run(["c++", "-std=c++17", "-O1", str(src), "-o", str(exe), "-pthread"], check=True)
+    assert subprocess.run([str(exe)], capture_output=True, timeout=60).returncode == 0
