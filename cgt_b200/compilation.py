@@ -91,8 +91,13 @@ class _SpecialisedByShape(object):
 
     Almost every graph rewrite needs to know extents: with an open batch extent a training step of a small network is
     30 launches and a dozen host instructions instead of 10 and none. So the third call with the same argument shapes
-    compiles the graph for them (tens of milliseconds) and later calls with these shapes go there; everything else, and
-    the first two calls with any shape, runs the general function. All copies read and update the same shared variables.
+    compiles the graph for them (tens of milliseconds for a small network whose generated kernels are in the cache, seconds
+    for every kernel that is not and for a long unrolled network) and later calls with these shapes go there; everything
+    else, and the first two calls with any shape, runs the general function. All copies read and update the same shared
+    variables. Their sums may be added up in another order than the general function's.
+
+    With several ranks nothing is compiled inside a call: the others would wait in their collective for the rank that
+    compiles, longer than the peer exchange's limit.
 
     At most MOST copies are kept, the least recently used one is dropped; each drop doubles the number of calls that earn
     a copy, so that a program which goes round many shapes soon runs the general function and compiles nothing. A copy
@@ -116,7 +121,8 @@ class _SpecialisedByShape(object):
             return None
 
     def _pick(self, args, count):
-        key = self._shapes(args)
+        from . import parallel
+        key = self._shapes(args) if parallel.world_size() == 1 else None
         if key is None or len(args) != len(self._source[0]):
             return self._general
         with self._lock:

@@ -578,6 +578,16 @@ def test_copies_per_shape_do_not_thrash(monkeypatch, n_shapes):
     assert f(np.zeros((99, 3), "f4")) == "general" and f([[1.0, 2.0]]) == "general"
 
 
+def test_nothing_is_compiled_inside_a_call_of_several_ranks(monkeypatch):
+    from cgt_b200 import parallel
+    monkeypatch.setattr(compilation, "run_compilation_pipeline", lambda *a: pytest.fail("compiled inside a call"))
+    monkeypatch.setattr(compilation._SpecialisedByShape, "_room", staticmethod(lambda: True))
+    monkeypatch.setitem(parallel._state, "world", 2)
+    x = cgt.matrix("x")
+    f = compilation._SpecialisedByShape(lambda *args: "general", [x], [x * 2.0], None, [])
+    assert {f(np.zeros((4, 3), "f4")) for _ in range(10)} == {"general"} and not f._copies
+
+
 def _gpu_ops(cfg):
     eg = compilation.execution_graph(cfg.inputs, [cfg.loss] + list(cfg.extra_outputs), cfg.updates, [])[0]
     return [i.op for i in eg.instrs if getattr(i, "op", None) is not None]
