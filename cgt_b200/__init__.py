@@ -3,12 +3,33 @@ Toolkit. The module namespace plays the role of the reference's ``cgt`` package:
 ``function``, ``grad``, configuration.
 """
 import sys as _sys
+import types as _types
 
 from . import core, utils
 from . import api as _api
 
-floatX = "f4"
-complexX = "c8"
+
+class _Package(_types.ModuleType):
+    """floatX and complexX are attributes of the package that depend on the thread (core.options_of_thread)."""
+
+    @property
+    def floatX(self):
+        return core.float_dtype()
+
+    @floatX.setter
+    def floatX(self, dtype):
+        core.floatX = dtype
+
+    @property
+    def complexX(self):
+        return {"f4": "c8", "f8": "c16"}[core.float_dtype()]
+
+    @complexX.setter
+    def complexX(self, dtype):
+        core.complexX = dtype
+
+
+_sys.modules[__name__].__class__ = _Package
 
 core.cgt = _sys.modules[__name__]
 _api.cgt = _sys.modules[__name__]

@@ -334,11 +334,7 @@ def reshape(x, shp):
 def set_precision(prec):
     """prec in {"single", "double"}: global float dtype."""
     assert prec in ("single", "double")
-    if prec == "single":
-        cgt.floatX, cgt.complexX = "f4", "c8"
-    else:
-        cgt.floatX, cgt.complexX = "f8", "c16"
-    core.floatX, core.complexX = cgt.floatX, cgt.complexX
+    core.floatX, core.complexX = ("f4", "c8") if prec == "single" else ("f8", "c16")
 
 
 def get_precision():

@@ -522,8 +522,13 @@ def generate_all(ops):
             todo.setdefault((type(op), sources[type(op)](op)), []).append(op)
     if not core.get_config().get("jit_fused_elementwise", True):
         return 0
+    (config, floatX) = (core.get_config(), core.float_dtype())
+
+    def make(op):
+        with core.options_of_thread(config, floatX):
+            return makers[type(op)](op)
     with concurrent.futures.ThreadPoolExecutor(8) as pool:
-        for (same, addr) in zip(todo.values(), pool.map(lambda same: makers[type(same[0])](same[0]), todo.values())):
+        for (same, addr) in zip(todo.values(), pool.map(lambda same: make(same[0]), todo.values())):
             n += len(same) if addr else 0
     return n
 

@@ -23,6 +23,7 @@ import string
 import subprocess
 import sys
 import threading
+import warnings
 from collections import defaultdict
 from io import StringIO
 
@@ -83,6 +84,9 @@ def _function_listout(inputs, outputs, dbg=None, updates=None, givens=None):
     if core.get_config()["specialise_shapes"] and any(None in inp.get_fixed_shape() for inp in inputs if is_tensor(inp)):
         return _SpecialisedByShape(f, inputs, outputs, updates, givens or [])
     return f
+
+
+_compiling_again = threading.Lock()
 
 
 class _SpecialisedByShape(object):
@@ -157,19 +161,17 @@ class _SpecialisedByShape(object):
         (inputs, outputs, updates, givens) = self._source
         if any(len(s) != inp.ndim for (s, inp) in zip(shapes, inputs)):
             return self._general     # it reports the error
-        config = core.get_config()
-        saved, floatX = dict(config), _cgt().floatX
+        if any(d is not None and int(d) != n for (s, inp) in zip(shapes, inputs) for (n, d) in zip(s, inp.get_fixed_shape())):
+            return self._general     # not the extents that were declared: whatever it does with them
         try:
-            config.update(self._config)   # the options that the function was compiled under
-            _cgt().set_precision("single" if self._floatX == "f4" else "double")
-            new = [core.Argument(inp.typ, name=inp.name, fixed_shape=tuple(int(d) for d in s), props=inp.props) for (s, inp) in zip(shapes, inputs)]
-            given = [(v, core.clone(w, dict(zip(inputs, new)))) for (v, w) in givens] + list(zip(inputs, new))
-            return run_compilation_pipeline(new, outputs, updates, given)
-        except Exception:   # extents that do not fit together: the general function reports that as it always did
+            with core.options_of_thread(self._config, self._floatX), _compiling_again:
+                new = [core.Argument(inp.typ, name=inp.name, fixed_shape=tuple(int(d) for d in s), props=inp.props) for (s, inp) in zip(shapes, inputs)]
+                given = [(v, core.clone(w, dict(zip(inputs, new)))) for (v, w) in givens] + list(zip(inputs, new))
+                return run_compilation_pipeline(new, outputs, updates, given)
+        except Exception as err:   # extents that do not fit together: the general function reports that as it always did
+            warnings.warn("compiling a function for argument shapes %s failed (%s: %s); the general one runs"
+                          % (shapes, type(err).__name__, err))
             return self._general
-        finally:
-            config.update(saved)
-            _cgt().set_precision("single" if floatX == "f4" else "double")
 
     def __call__(self, *args):
         return self._pick(args, True)(*args)

@@ -13,6 +13,7 @@ import hashlib
 import math
 import os
 import pickle
+import threading
 import traceback
 from collections import defaultdict, namedtuple
 from functools import reduce
@@ -432,8 +433,9 @@ def as_node(val_or_node):
 
 
 def default_props():
-    props = {"default_device": _CONFIG["default_device"]}
-    if _CONFIG["debug"]:
+    config = get_config()
+    props = {"default_device": config["default_device"]}
+    if config["debug"]:
         props["stack"] = traceback.extract_stack()[:-3]
     return props
 
@@ -2501,10 +2503,35 @@ _DEFAULTS = dict(
 )
 
 _CONFIG = None
+_of_thread = threading.local()
+
+
+class options_of_thread(object):
+    """``with options_of_thread(config, floatX): ...``: within the block get_config() and cgt.floatX are these, for the
+    calling thread only. A function that compiles again later does so under the options of its first compilation, while
+    other threads build graphs and compile under theirs."""
+
+    def __init__(self, config, floatX):
+        self.options = (dict(config), floatX)
+
+    def __enter__(self):
+        self.outer = getattr(_of_thread, "options", None)
+        _of_thread.options = self.options
+
+    def __exit__(self, *args):
+        _of_thread.options = self.outer
+
+
+def float_dtype():
+    options = getattr(_of_thread, "options", None)
+    return floatX if options is None else options[1]
 
 
 def get_config(force_reload=False):
     global _CONFIG
+    options = getattr(_of_thread, "options", None)
+    if options is not None and not force_reload:
+        return options[0]
     if _CONFIG is None or force_reload:
         _CONFIG = _load_config()
     return _CONFIG

@@ -588,6 +588,40 @@ def test_nothing_is_compiled_inside_a_call_of_several_ranks(monkeypatch):
     assert {f(np.zeros((4, 3), "f4")) for _ in range(10)} == {"general"} and not f._copies
 
 
+def test_a_copy_is_compiled_under_its_functions_options_and_nobody_elses(monkeypatch):
+    """While a copy is compiled, in single precision and without fusion, another thread sees double precision and fusion;
+    afterwards everything is as before. What goes wrong is said, and the general function runs."""
+    import threading
+    seen, other = {}, {}
+
+    def look():
+        other.update(floatX=cgt.floatX, fuse=core.get_config()["fuse_elementwise"], arg=cgt.matrix("z").dtype)
+
+    def compiler(inputs, *_rest):
+        seen.update(floatX=cgt.floatX, fuse=core.get_config()["fuse_elementwise"], arg=cgt.matrix("z").dtype)
+        t = threading.Thread(target=look)
+        t.start()
+        t.join()
+        raise ValueError("not a dag")
+    monkeypatch.setattr(compilation, "run_compilation_pipeline", compiler)
+    monkeypatch.setattr(compilation._SpecialisedByShape, "_room", staticmethod(lambda: True))
+    with cgt.scoped_update_config(fuse_elementwise=False):
+        x = cgt.matrix("x", fixed_shape=(None, 3))
+        f = compilation._SpecialisedByShape(lambda *args: "general", [x], [x * 2.0], None, [])
+    with cgt.scoped_update_config(precision="double"):
+        for _ in range(2):
+            f(np.zeros((4, 3), "f4"))
+        with pytest.warns(UserWarning, match="not a dag"):
+            assert f(np.zeros((4, 3), "f4")) == "general"
+        assert seen == dict(floatX="f4", fuse=False, arg="f4") and other == dict(floatX="f8", fuse=True, arg="f8")
+        assert cgt.floatX == "f8" and core.get_config()["fuse_elementwise"]
+        seen.clear()
+        for _ in range(5):   # not the declared extents: nothing is compiled for them
+            assert f(np.zeros((4, 2), "f4")) == "general"
+        assert not seen
+    assert cgt.floatX == "f4" == core.floatX
+
+
 def _gpu_ops(cfg):
     eg = compilation.execution_graph(cfg.inputs, [cfg.loss] + list(cfg.extra_outputs), cfg.updates, [])[0]
     return [i.op for i in eg.instrs if getattr(i, "op", None) is not None]
