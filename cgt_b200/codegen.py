@@ -550,6 +550,7 @@ def _product_header():
 def _generated_launcher(src, tag, symbol, what):
     import ctypes
     import os.path as osp
+    import threading
     from . import compilation, utils
     if not core.get_config().get("jit_fused_elementwise", True):
         return None
@@ -560,13 +561,15 @@ def _generated_launcher(src, tag, symbol, what):
     libpath = osp.join(info["CACHE_ROOT"], prefix + ".so")
     try:
         if not osp.exists(libpath):
-            srcpath = osp.join(info["CACHE_ROOT"], prefix + ".cu")
-            with open(srcpath, "w") as fh:
+            # files of this thread's own until they are complete: other ranks and threads may want the same kernel
+            (srcpath, mine) = (osp.join(info["CACHE_ROOT"], prefix + ".cu"), "%d.%d" % (os.getpid(), threading.get_ident()))
+            with open("%s.%s.cu" % (srcpath, mine), "w") as fh:
                 fh.write(src)
-            compilation._call("nvcc %s -o %s.tmp -shared -gencode arch=compute_100a,code=sm_100a -lineinfo -O3 -std=c++17 "
+            compilation._call("nvcc %s.%s.cu -o %s.%s.tmp -shared -gencode arch=compute_100a,code=sm_100a -lineinfo -O3 -std=c++17 "
                               "-fmad=false -Xcompiler -fPIC %s -L/usr/local/cuda/lib64 -lcudart"
-                              % (srcpath, libpath, info["INCLUDES"]))
-            os.replace(libpath + ".tmp", libpath)
+                              % (srcpath, mine, libpath, mine, info["INCLUDES"]))
+            os.replace("%s.%s.cu" % (srcpath, mine), srcpath)
+            os.replace("%s.%s.tmp" % (libpath, mine), libpath)
         lib = ctypes.CDLL(libpath)
         addr = ctypes.cast(getattr(lib, symbol), ctypes.c_void_p).value
     except (RuntimeError, OSError) as err:

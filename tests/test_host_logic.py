@@ -730,3 +730,30 @@ def test_copies_without_helper_threads(tmp_path):
     src.write_text(_COPY_LIMIT % osp.join(ROOT, "cgt_b200", "csrc"))
     subprocess.run(["c++", "-std=c++17", "-O1", str(src), "-o", str(exe), "-pthread"], check=True)
     assert subprocess.run([str(exe)], capture_output=True, timeout=60).returncode == 0
+
+
+def test_two_threads_compile_one_kernel_into_files_of_their_own(tmp_path, monkeypatch, capsys):
+    """Neither the source that a compiler reads nor the library that it writes may be another compiler's."""
+    import shlex
+    import threading
+    from cgt_b200 import codegen
+    (both, files) = (threading.Barrier(2, timeout=30), [])
+
+    def compiler(cmd):
+        both.wait()
+        words = shlex.split(cmd)
+        (src, out) = (words[1], words[words.index("-o") + 1])
+        files.append((src, out))
+        assert open(src).read() == "// a kernel"
+        open(out, "w").write("not a library")
+        both.wait()
+    monkeypatch.setattr(compilation, "get_compile_info", lambda: dict(CACHE_ROOT=str(tmp_path), INCLUDES=""))
+    monkeypatch.setattr(compilation, "_call", compiler)
+    monkeypatch.setattr(codegen, "_fused_libs", {})
+    threads = [threading.Thread(target=codegen._generated_launcher, args=("// a kernel", "test_", "none", "a test")) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(files) == 2 and len({f for pair in files for f in pair}) == 4
+    assert sorted(f.rsplit(".", 1)[1] for f in os.listdir(str(tmp_path))) == ["cu", "so"]
