@@ -187,7 +187,8 @@ int product_fma_t(const Product<T>& q, bool tiles_only) {
 
 bool product_is_fma(int tA, int tB, long P, long M, long N, long K) {
   if (warp_per_output(tA, tB, M, N) && small_shape(P, M, N, K)) return true;
-  return P * M * N * K <= (1L << 26);
+  if (P > 65535) return false;  // one grid layer per product
+  return M * N * K <= (1L << 25) || P * M * N * K <= (1L << 26);
 }
 int product_fma(const Product<float>& q, bool tiles_only) { return product_fma_t(q, tiles_only); }
 int product_fma(const Product<double>& q, bool tiles_only) { return product_fma_t(q, tiles_only); }

@@ -34,7 +34,9 @@ struct Product {
 
 // The FMA kernels take a product below the size at which the tensor-core kernels' fixed cost (tensor-map fetch,
 // tensor-memory allocation, a ring that a short K never fills: 10 - 15 us, 2 us more for the fold of a split K) is
-// repaid: 39 M multiplications 8.4 and 15 us, 107 M (3200 x 512 x 65) 22 and 14 us.
+// repaid: 39 M multiplications 8.4 and 15 us, 107 M (3200 x 512 x 65) 22 and 14 us. A batch of products of up to 2^25
+// multiplications each stays with them whatever its length: 128 of 256^3 take 163 us here and 61 us on the tensor cores,
+// but the three-fold TF32 split is off by 1.3e-6 (2-norm, against 64 bits) where plain float32 is off by 1.5e-7.
 bool product_is_fma(int tA, int tB, long P, long M, long N, long K);
 // 0 done, 1 error, -1: `chain` was compiled for another variant than this product needs. tiles_only: no small-product kernel
 int product_fma(const Product<float>& q, bool tiles_only = false);

@@ -59,3 +59,15 @@ def test_chains_in_the_output_stage_change_no_bit(rt, B, xdim, hidden):
         results[on] = [np.asarray(v).copy() for _ in range(4) for v in f(xs)] + [p.op.get_value() for p in (W, b, V)]
     for (p, q) in zip(results[False], results[True]):
         assert np.array_equal(p, q)
+
+
+@pytest.mark.parametrize("P,M,N,K", [(64, 64, 64, 64), (512, 64, 64, 64), (16, 256, 256, 128), (128, 256, 256, 256), (70, 100, 100, 1000)])
+def test_batched_products_are_plain_float32(rt, P, M, N, K):
+    """A chain of K rounded additions of random terms is off by u * sqrt(K / 6) (2-norm, u = 2^-24), half as much again for
+    its spread; the TF32 split of the tensor-core kernels is off by more. Long batches and short ones alike."""
+    rs = np.random.RandomState(0)
+    (A, B) = (rs.randn(P, M, K).astype("f4"), rs.randn(P, K, N).astype("f4"))
+    (dA, dB, dC) = (Dev(A), Dev(B), Dev(np.zeros((P, M, N), "f4")))
+    call("cgtb_sgemm_batched", 0, 0, P, M, N, K, dA.ptr, K, M * K, dB.ptr, N, K * N, dC.ptr, N, M * N, 0)
+    want = A.astype("f8") @ B.astype("f8")
+    assert np.linalg.norm(dC.get() - want) <= 1.5 * 2.0 ** -24 * np.sqrt(K / 6.0) * np.linalg.norm(want)
