@@ -53,7 +53,7 @@ class HostRun(object):
         self.variables = {}
         for node in core.topsorted(list(outputs) + [n for (_v, n) in updates] + [v for (v, _n) in updates]):
             if node.is_data():
-                self.variables[node.op] = np.ascontiguousarray(node.op.get_value()).copy()
+                self.variables[node.op] = np.array(node.op.get_value(), order="C", copy=True)
         (self.eg, outs, memloc) = compilation.execution_graph(list(inputs), list(outputs), list(updates), [])
         self.out_locs = [memloc[o].index for o in outs]
         self._oracle = cpu_backend.OracleFunction([], [])

@@ -167,3 +167,25 @@ def test_a_slice_that_is_handed_out_keeps_its_old_value():
     assert not any(isinstance(op, core.LeadingSlice) for op in run.ops())
     run = _same_as_oracle([], [cgt.tanh(W[2:5])], [(W, W * 0.9)])
     assert any(isinstance(op, core.LeadingSlice) for op in run.ops())
+
+
+@pytest.mark.parametrize("delay", [True, False])
+def test_host_arithmetic_behind_the_device_work(delay):
+    """Steps scaled by several norms that the host works out, a host variable that the host overwrites, and the order of
+    what reads and writes it: the same bits wherever the host's instructions stand, and one stretch of them when delayed."""
+    from cgt_b200 import compilation
+    rs = np.random.RandomState(0)
+    x = cgt.matrix("x", fixed_shape=(33, 5))
+    (a, b, p) = (_var(rs, 33, 5), _var(rs, 33, 5), _var(rs, 33, 5))
+    lr = cgt.shared(np.array(0.25, "f4"), device=core.Device("cpu", 0))
+    with cgt.scoped_update_config(delay_host_arithmetic=delay, fuse_square_sums=False):
+        norms = [cgt.sqrt(cgt.square(v * x).sum()) for v in (a, b, p)]
+        scale = lr / (norms[0] + norms[1] * norms[2])
+        run = _same_as_oracle([x], [norms[1] * 2.0, lr * 1.0 + norms[0]],
+                              [(a, a - scale * x), (b, b - norms[0] * lr * x), (p, p - x), (lr, lr * 0.5 + 0.0 * norms[2])])
+    instrs = [i for i in run.eg.instrs if isinstance(i, compilation.ReturnByRef) and not i.once and not isinstance(i.op, core.Constant)]
+    downloads = [i for i in instrs if isinstance(i.op, core.Transport) and i.write_loc.devtype == "cpu"]
+    roots = [k for (k, i) in enumerate(instrs) if getattr(i.op, "opname", "") == "sqrt"]
+    assert len(downloads) == 3 and len(roots) == 3
+    (first, last) = (min(roots), max(instrs.index(d) for d in downloads))
+    assert (first > last) == delay
