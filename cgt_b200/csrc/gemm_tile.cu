@@ -209,8 +209,7 @@ int product_small(const Product<float>& q) {
   return run_product<float>(q, pl);
 }
 int product_variant(int dtype, int tA, int tB, long M, long N, long K) {
-  if (M <= 0 || N <= 0) return -1;
-  if (dtype == cgtb_f8) return plan_product<double>(tA, tB, 1, M, N, K, true).plan.variant;
+  if (dtype != cgtb_f4 || M <= 0 || N <= 0) return -1;
   return product_is_fma(tA, tB, 1, M, N, K) ? plan_product<float>(tA, tB, 1, M, N, K, true).plan.variant : -1;
 }
 

@@ -352,24 +352,16 @@ OP_BYREF(cgtb_op_mul22_chain) {
   long bk[CGTB_FUSED_MAX_IN], binner[CGTB_FUSED_MAX_IN], n;
   if (!chain_operands(&cl->chain, reads + 2, write0, cl->product, &n, in, bk, binner, out)) return;
   if (n != M * N) { fail("Mul22Chain: the chain's results have %ld elements, the product %ld", n, M * N); return; }
+  if (A->dtype() != cgt_f4) { fail("Mul22Chain: unsupported dtype %d", (int)A->dtype()); return; }
   const Chain chain = {(ChainLauncher)cl->launcher, cl->variant, in, bk, binner, out};
-  auto go = [&](auto* tag) {
-    typedef typename std::remove_pointer<decltype(tag)>::type T;
-    Product<T> q = {cl->tA, cl->tB, 1, M, N, K, (const T*)A->data(), lda, 0, (const T*)B->data(), ldb, 0, nullptr, N, 0};
-    q.chain = &chain;
-    int rc = cl->launcher ? product_fma(q) : -1;
-    if (rc >= 0) return;
-    // no kernel was generated, or the extents are not those it was generated for
-    T* c = (T*)scratch_outer((size_t)n * sizeof(T));
-    if (!c) return;
-    if constexpr (sizeof(T) == 4) rc = sgemm_dispatch(cl->tA, cl->tB, 1, M, N, K, q.A, lda, 0, q.B, ldb, 0, c, N, 0, 0);
-    else rc = cgtb_dgemm(cl->tA, cl->tB, M, N, K, q.A, lda, q.B, ldb, c, N);
-    if (rc) return;
-    in[cl->product] = c;
-    cgtb_fused_elwise(&fp, n, in, bk, binner, out);
-  };
-  if (A->dtype() == cgt_f4) go((float*)nullptr);
-  else fail("Mul22Chain: unsupported dtype %d", (int)A->dtype());
+  Product<float> q = {cl->tA, cl->tB, 1, M, N, K, (const float*)A->data(), lda, 0, (const float*)B->data(), ldb, 0, nullptr, N, 0};
+  q.chain = &chain;
+  if (cl->launcher && product_fma(q) >= 0) return;
+  // no kernel was generated, or the extents are not those it was generated for
+  float* c = (float*)scratch_outer((size_t)n * sizeof(float));
+  if (!c || sgemm_dispatch(cl->tA, cl->tB, 1, M, N, K, q.A, lda, 0, q.B, ldb, 0, c, N, 0, 0)) return;
+  in[cl->product] = c;
+  cgtb_fused_elwise(&fp, n, in, bk, binner, out);
 }
 // Mul22BiasAdd: (A, B, bias [1,N], addend [M,N], addend_bias [1,N]) -> (addend + addend_bias) + (A.B + bias)
 OP_BYREF(cgtb_op_mul22_bias_add) {

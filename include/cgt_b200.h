@@ -164,8 +164,8 @@ int cgtb_sgemm_batched(int tA, int tB, long P, long M, long N, long K, const flo
  * kernel (M*N > 2048, M*N*K <= 2^26, not A.B^T); others are refused. */
 int cgtb_sgemm_bias_add(int tA, int tB, long M, long N, long K, const float* A, long lda, const float* B, long ldb,
                         const float* bias, const float* addend, long ldd, const float* addend_bias, float* C, long ldc);
-/* Which of the FMA product kernels (cgt_product.h) this product runs in, -1 when it goes to the tensor cores; what an
- * elementwise chain in its output stage is compiled for. */
+/* Which of the FMA product kernels (cgt_product.h) this product runs in, what an elementwise chain in its output stage is
+ * compiled for; -1 when it goes to the tensor cores, or is not float32: chains are float32. */
 int cgtb_product_variant(int dtype, int tA, int tB, long M, long N, long K);
 int cgtb_dgemm(int tA, int tB, long M, long N, long K, const double* A, long lda, const double* B, long ldb,
                double* C, long ldc);
