@@ -277,12 +277,14 @@ def _foldable_repeat(node):
 
 def variables_seen(node):
     """The shared variables whose memory `node` is or views."""
+    if node.op is not None and node.op.return_type != "byval":
+        return frozenset()
     (found, stack) = (set(), [node])
     while stack:
         n = stack.pop()
         if n.is_data():
             found.add(n)
-        elif not n.is_input() and n.op.return_type == "byval" and not isinstance(n.op, core.Size):
+        elif n.op is not None and n.op.return_type == "byval" and not isinstance(n.op, core.Size):
             stack.extend(n.parents)
     return found
 
@@ -290,9 +292,12 @@ def variables_seen(node):
 def variables_read(node):
     """The shared variables whose memory the operation of `node` reads; operands of which only the extents count are none."""
     if node.is_input():
-        return set()
+        return frozenset()
+    seen = [(pos, vs) for (pos, vs) in enumerate(map(variables_seen, node.parents)) if vs]
+    if not seen:
+        return frozenset()
     skip = _meta_inputs(node.op, len(node.parents))
-    return set().union(*[variables_seen(par) for (pos, par) in enumerate(node.parents) if pos not in skip])
+    return set().union(*[vs for (pos, vs) in seen if pos not in skip])
 
 
 class UpdateOrder(object):
@@ -304,7 +309,12 @@ class UpdateOrder(object):
     one from now on."""
 
     def __init__(self, outputs, updatetargs, updatesrcs):
-        nodes = core.topsorted(list(outputs) + list(updatetargs))
+        self.step = (list(outputs), list(updatetargs), list(updatesrcs))
+        self.later = None
+
+    def _find(self):
+        (outputs, updatetargs, updatesrcs) = self.step
+        nodes = core.topsorted(outputs + updatetargs)
         number = {t: i for (i, t) in enumerate(updatetargs)}
         target_of = dict(zip(updatesrcs, updatetargs))
         self.later = defaultdict(list)
@@ -320,6 +330,8 @@ class UpdateOrder(object):
                     self.later[node].append(t)
 
     def closes_cycle(self, group):
+        if self.later is None:
+            self._find()
         (group, seen) = (set(group), set())
         stack = [n for m in group for n in self.later[m] if n not in group]
         while stack:
@@ -332,6 +344,8 @@ class UpdateOrder(object):
         return False
 
     def join(self, group):
+        if self.later is None:
+            self._find()
         for (a, b) in zip(group[:-1], group[1:]):
             self.later[a].append(b)
             self.later[b].append(a)
@@ -2827,10 +2841,10 @@ def merge_parameter_updates(eg, update_locs):
             held.update(*[holds[r.index] for r in ins.read_locs if r.index in holds])
 
     def memory(locs):
-        return set().union(*[holds[loc.index] for loc in locs]) if locs else set()
+        return set().union(*[holds[loc.index] for loc in locs])
 
     def written_by(ins):
-        if isinstance(ins, (ReturnByVal, BuildTup, Alloc, LoadArgument)):
+        if not isinstance(ins, ReturnByRef):
             return set()
         extra = ins.read_locs[len(ins.read_locs) - ins.op.k + 1:] if isinstance(ins.op, core.MultiFusedElwise) else []
         return memory([ins.write_loc] + list(extra))
@@ -2849,12 +2863,15 @@ def merge_parameter_updates(eg, update_locs):
     # parameter's own update) have moved to the end, the chains that write it can move past their old readers
     for (key, idxs) in sorted(groups.items(), key=lambda kv: -kv[1][-1]):
         last = idxs[-1]
-        movable = []
-        for i in idxs:
-            result, reads = written_by(instrs[i]), memory(instrs[i].read_locs)
-            if all(not (result & memory(list(getattr(instrs[j], "read_locs", [])) + [instrs[j].write_loc])) and
-                   not (reads & written_by(instrs[j])) for j in range(i + 1, last + 1)):
-                movable.append(i)
+        movable, touched, written = [], set(), set()    # by the instructions behind the one looked at
+        for j in range(last, idxs[0] - 1, -1):
+            ins = instrs[j]
+            (result, reads) = (written_by(ins), memory(getattr(ins, "read_locs", [])))
+            if j in idxs and not (result & touched) and not (reads & written):
+                movable.append(j)
+            touched |= result | reads | holds[ins.write_loc.index]
+            written |= result
+        movable.reverse()
         movable = movable[:24]
         if len(movable) < 2:
             continue
