@@ -338,8 +338,9 @@ def recurrence_plan(R, H, KA, N, n_act):
         KG = -(-KA // KT)
         RB = -(-R // (128 // C))
         shared = 4 * (2 * RB * KG * KT + KG * RB * NC)
-        # 72 weights per thread leave registers for the sums and the chain; 8 rows: beyond that, a launch per step over
-        # the whole batch has enough work per block
+        # 72 weights per thread leave registers for the sums and the chain. A thread per (row, unit) runs the chain, which ends
+        # most plans: at 8 rows of 32 units a training step over 1024 examples takes 403 us, as separate launches 511. With
+        # fewer units the limit of 8 rows ends them, which was not measured
         if KT > 72 or RB > 8 or RB * UH > 256 or shared > 46 * 1024:
             continue
         if best is None or RB * KT < best[0]:
