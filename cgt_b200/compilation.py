@@ -109,6 +109,8 @@ class _SpecialisedByShape(object):
     MOST, AFTER, WATCHED = 4, 3, 64
 
     def __init__(self, general, inputs, outputs, updates, givens):
+        from . import parallel
+        self._world_size = parallel.world_size
         self._general = general
         self._source = (inputs, outputs, updates, givens)
         self._config = dict(core.get_config())
@@ -125,8 +127,7 @@ class _SpecialisedByShape(object):
             return None
 
     def _pick(self, args, count):
-        from . import parallel
-        key = self._shapes(args) if parallel.world_size() == 1 else None
+        key = self._shapes(args) if self._world_size() == 1 else None
         if key is None or len(args) != len(self._source[0]):
             return self._general
         with self._lock:
