@@ -2565,6 +2565,27 @@ def _in_place_unsafe(node):
     return [pos for (pos, par) in enumerate(node.parents) if pos < product or not whole(par)]
 
 
+def _copy(node):
+    """Result node: the elements of `node` in memory of their own."""
+    name = "cast_to_" + node.dtype
+    return core.Result(core.ElwiseUnary(name, core.UnaryInfo(name, None, False, node.dtype, None, "x")), [node])
+
+
+def copy_shared_targets(updatetargs, node2shape):
+    """An update target is computed in its variable's memory: one instruction per variable. A value that several variables
+    get, and one that is a view of something else (a reshape, some rows), is copied into the variable."""
+    (out, seen) = ([], set())
+    for t in updatetargs:
+        if t in seen or (not t.is_input() and t.op.return_type == "byval"):
+            copy = _copy(t)
+            copy.props.update(t.props)
+            node2shape[copy] = node2shape[t]
+            t = copy
+        seen.add(t)
+        out.append(t)
+    return out
+
+
 def keep_old_values(outputs_all, updates, node2dev, node2shape):
     """Every operation sees the variables as they were before the call: an operation that reads a variable and cannot run
     before the variable's update, because it needs the new value too or because two updates need each other's variable,
@@ -2585,11 +2606,7 @@ def keep_old_values(outputs_all, updates, node2dev, node2shape):
             if node is not v and (node.is_input() or v not in variables_seen(node)):
                 return node
             if node not in copies:
-                if node is v:
-                    name = "cast_to_" + v.dtype
-                    new = core.Result(core.ElwiseUnary(name, core.UnaryInfo(name, None, False, v.dtype, None, "x")), [v])
-                else:
-                    new = core.Result(node.op, [old(par) for par in node.parents], typ=node.typ)
+                new = _copy(v) if node is v else core.Result(node.op, [old(par) for par in node.parents], typ=node.typ)
                 new.props.update(node.props)
                 (node2dev[new], node2shape[new]) = (node2dev[node], node2shape[node])
                 copies[node] = new
@@ -2969,6 +2986,7 @@ def execution_graph(inputs, outputs, updates, givens):
     config = core.get_config()
     outputs_simple, updatesrcs, updatetargs_simple, analysis = simplify_for_execution(outputs, updates, givens)
     node2shape = analysis["node2shape"]
+    updatetargs_simple = copy_shared_targets(updatetargs_simple, node2shape)
     outputs_simple, updatetargs_simple = rewrite_for_execution(outputs_simple, updatetargs_simple, updatesrcs, node2shape)
     all_out = outputs_simple + updatetargs_simple
 

@@ -189,3 +189,14 @@ def test_host_arithmetic_behind_the_device_work(delay):
     assert len(downloads) == 3 and len(roots) == 3
     (first, last) = (min(roots), max(instrs.index(d) for d in downloads))
     assert (first > last) == delay
+
+
+def test_one_value_for_several_variables_and_views_as_values():
+    rs = np.random.RandomState(0)
+    (a, b, c) = (_var(rs, 6, 6), _var(rs, 6, 6), _var(rs, 6, 6))
+    x = cgt.matrix("x", fixed_shape=(6, 6))
+    y = cgt.matrix("y", fixed_shape=(4, 9))
+    new = a + x * b
+    _same_as_oracle([x], [c - new], [(a, new), (b, new), (c, new)])
+    _same_as_oracle([y], [a * 2.0], [(a, cgt.tanh(y).reshape([6, 6]))])
+    _same_as_oracle([], [a * 2.0, b * 3.0], [(a, cgt.concatenate([b, b], axis=0)[3:9]), (b, b - a)])
