@@ -34,6 +34,13 @@ def _own_rows(rs):
     return [A, x], [], [(W, W - 0.1 * A.dot(W[16:32])), (last, cgt.concatenate([x, last[0:7]], axis=0))]
 
 
+def _views_and_shared_values(rs):
+    x = cgt.matrix("x", fixed_shape=(64, 40))
+    (a, b, c, d) = (_var(rs, 64, 40), _var(rs, 64, 40), _var(rs, 40, 64), _var(rs, 16, 40))
+    new = 0.5 * a + x * b
+    return [x], [cgt.tanh(c), d * 2.0], [(a, new), (b, new), (c, cgt.tanh(x + a).reshape([40, 64])), (d, cgt.tanh(x)[8:24])]
+
+
 def _each_other(rs):
     g = cgt.matrix("g", fixed_shape=(333, 50))
     (v, p, d) = (_var(rs, 333, 50), _var(rs, 333, 50), _var(rs, 333, 50))
@@ -50,7 +57,7 @@ def _optimizer(name):
     return build
 
 
-@pytest.mark.parametrize("build", [_factorisation, _old_and_new, _own_rows, _each_other, _optimizer("momentum"), _optimizer("nesterov_momentum"),
+@pytest.mark.parametrize("build", [_factorisation, _old_and_new, _own_rows, _views_and_shared_values, _each_other, _optimizer("momentum"), _optimizer("nesterov_momentum"),
                                    _optimizer("rmsprop"), _optimizer("adadelta")])
 def test_against_the_oracle(rt, build):
     (inputs, outputs, updates) = build(np.random.RandomState(0))
